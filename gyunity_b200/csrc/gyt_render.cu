@@ -655,7 +655,9 @@ GYT_D void gen_path(PathBuf& dst, uint32_t k, uint32_t x, uint32_t y, uint32_t s
   const bool halton = cam.sampler != 0;
   uint64_t idx = halton ? halton_enum_index(cam, s, x, y) : enum_index(tab, cam.log2_res, s, x, y);
   Rng rng{idx, 0};
-  float su = rng.next(tab, cam.sampler), sv = rng.next(tab, cam.sampler);
+  float uv[2];
+  rng.next<2>(tab, cam.sampler, uv);
+  const float su = uv[0], sv = uv[1];
   // SobolEnum::SampleX/Y (SobolEnum.h:30-36) or HaltonEnum::scale_x/y, kept
   // unfused as the reference
   float u = __fsub_rn(__fmul_rn(halton ? cam.h_sx : cam.res_pow2, su), (float)x);
@@ -854,8 +856,7 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
     // arguments in GCC's right-to-left order: v.z v.y v.x u.y u.x uLight), three
     // for the BSDF sample (PT.cpp:47, again z y x) and one for roulette
     float u10[10];
-    if (SAMPLER == 1 || (SAMPLER < 0 && prm.sampler)) halton10(tab, rng.index, rng.cursor, u10);
-    else sobol10(tab.bits, rng.index, rng.cursor, u10);
+    rng.peek<10>(tab, SAMPLER < 0 ? prm.sampler : (uint32_t)SAMPLER, u10);
     const bool emit = (depth == 0 || delta) && light >= 0;
     // the continuation's four dimensions (arguments again in right-to-left
     // order) wait in shared memory while direct lighting runs: four registers
@@ -1682,9 +1683,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_light_trace(DevScene s, LtCam c, 
     if (s.n_area <= 0) continue;
     Rng rng{g, 0};
     // GCC evaluates the arguments right to left: light choice, then v (y, x), then u (y, x)
-    const float ul = rng.next(tab, prm.sampler);
-    const float vy = rng.next(tab, prm.sampler), vx = rng.next(tab, prm.sampler);
-    const float uy = rng.next(tab, prm.sampler), ux = rng.next(tab, prm.sampler);
+    float u5[5];
+    rng.next<5>(tab, prm.sampler, u5);
+    const float ul = u5[0], vy = u5[1], vx = u5[2], uy = u5[3], ux = u5[4];
     float lsel = 0.f;
     const int li = sample_light(s, ul, &lsel);
     if (li >= s.n_area) continue;  // environment light (rejected on the host)
@@ -1768,10 +1769,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_light_trace(DevScene s, LtCam c, 
       }
       ++bounce;
       if (bounce >= prm.max_depth) break;
-      const float rz = rng.next(tab, prm.sampler), ry = rng.next(tab, prm.sampler), rx = rng.next(tab, prm.sampler);
+      float u3[3];  // z, y, x
+      rng.next<3>(tab, prm.sampler, u3);
       float3 wi;
       float pdf;
-      const float3 f = bsdf.sample(h.wo, &wi, &pdf, rx, ry, rz);
+      const float3 f = bsdf.sample(h.wo, &wi, &pdf, u3[2], u3[1], u3[0]);
       if (pdf == 0.f) break;  // the reference continues with an undefined direction here
       o = (h.pos + wi * kRayEps) + wi * kRayEps;
       d = wi;
@@ -2031,7 +2033,7 @@ GYT_D void vpt_direct_queue(const DevScene& s, const Queues& q, const VPoint& p,
 // connection to that point (ConnectToLight, VPT.cpp:108-146), queued as a
 // shadow segment. The light point is recomputed from its two numbers where it
 // is used rather than kept.
-template <int W, bool EQUI>
+template <int SAMPLER, bool EQUI>
 __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, uint32_t n, DevScene s, Params prm,
                                                                  Queues q, SamplerTables tab) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2050,7 +2052,7 @@ __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, ui
   uint32_t crossings = __float_as_uint(d4.w);
   float3 tp = f3(cur.tp[i]);
   float3 nd = d;
-  const uint32_t dim_limit = prm.sampler ? kHaltonDims : 1024u;
+  const uint32_t dim_limit = SAMPLER ? kHaltonDims : 1024u;
   bool end = rng.cursor + 16u > dim_limit;  // the sampler's dimensions are spent
   if (!end) {
     bool scattered = false;
@@ -2061,15 +2063,19 @@ __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, ui
     if (EQUI) {
       // VPT.cpp:23-24: Scene::SampleOneLight, then SampleOnePoint's
       // Vec2(rand(), rand()) in right-to-left order
-      const float ul = rng.next(tab, prm.sampler);
-      euy = rng.next(tab, prm.sampler);
-      eux = rng.next(tab, prm.sampler);
-      eli = sample_light(s, ul, &elsel);
+      // and, in a medium, the distance's number after them
+      float u4[4];
+      rng.peek<4>(tab, SAMPLER, u4);
+      rng.cursor += 3;
+      euy = u4[1];
+      eux = u4[2];
+      eli = sample_light(s, u4[0], &elsel);
       if (medium >= 0) {
         // HomogeneousMedium::EquiAngularSampling (volume/Homogeneous.cpp:38-64)
         const MediumDev md = load_medium(s, medium);
         g = md.g;
-        const float u = rng.next(tab, prm.sampler);
+        const float u = u4[3];
+        rng.cursor += 1;
         const float3 lpos = light_point(load_light(s, eli), eux, euy).pos;
         const float dl = dot(lpos - o, d);
         const float D = length(o + d * dl - lpos);
@@ -2091,7 +2097,9 @@ __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, ui
       // HomogeneousMedium::Sample (volume/Homogeneous.cpp:12-30)
       const MediumDev md = load_medium(s, medium);
       g = md.g;
-      const float uc = rng.next(tab, prm.sampler), ud = rng.next(tab, prm.sampler);
+      float u2[2];
+      rng.next<2>(tab, SAMPLER, u2);
+      const float uc = u2[0], ud = u2[1];
       const int ch = min((int)(uc * 3.f), 2);
       const float sc = ch == 0 ? md.st.x : (ch == 1 ? md.st.y : md.st.z);
       const float dist = -logf(1.f - ud) / sc;
@@ -2152,6 +2160,11 @@ __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, ui
         }
       }
     }
+    // the numbers of the rest of the bounce at once: six for direct light
+    // (uLight last), then the continuation's three (surface) or two (medium)
+    float u9[9];
+    if (!end && !pass) rng.peek<9>(tab, SAMPLER, u9);
+    bool direct = false;
     if (EQUI && gather && scattered) {
       // VPT.cpp:36: the connection to the bounce's light point
       // (ConnectToLight, VPT.cpp:108-146) as a shadow segment
@@ -2170,21 +2183,21 @@ __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, ui
       }
     } else if (gather) {
       // one call site for surface and medium points
-      const float vz = rng.next(tab, prm.sampler), vy = rng.next(tab, prm.sampler), vx = rng.next(tab, prm.sampler);
-      const float uy = rng.next(tab, prm.sampler), ux = rng.next(tab, prm.sampler);
-      const float ul = rng.next(tab, prm.sampler);
-      vpt_direct_queue(s, q, p, scattered ? nullptr : &bsdf, g, tp, i, ul, ux, uy, vx, vy, vz);
+      direct = true;
+      rng.cursor += 6;
+      vpt_direct_queue(s, q, p, scattered ? nullptr : &bsdf, g, tp, i, u9[5], u9[4], u9[3], u9[2], u9[1], u9[0]);
     }
     if (!end && !pass) {
+      const float rz = direct ? u9[6] : u9[0], ry = direct ? u9[7] : u9[1], rx = direct ? u9[8] : u9[2];
       if (scattered) {
-        const float py = rng.next(tab, prm.sampler), px = rng.next(tab, prm.sampler);
+        rng.cursor += 2;
         float3 wi;
-        phase_sample(g, -d, px, py, &wi);
+        phase_sample(g, -d, ry, rz, &wi);
         o = mpos + wi * kRayEps;  // MediumIntersection::SpawnRay: no offset
         nd = wi;
         delta = false;
       } else {
-        const float rz = rng.next(tab, prm.sampler), ry = rng.next(tab, prm.sampler), rx = rng.next(tab, prm.sampler);
+        rng.cursor += 3;
         float3 wi;
         float pdf;
         const float3 f = bsdf.sample(p.wo, &wi, &pdf, rx, ry, rz);
@@ -2406,11 +2419,13 @@ __global__ void k_bsdf_table(uint64_t n, const float* __restrict__ params, const
   o[7] = fe.x; o[8] = fe.y; o[9] = fe.z; o[10] = pe;
 }
 
-__global__ void k_sobol(const uint32_t* __restrict__ mat, uint64_t n, const uint32_t* dims, const uint64_t* idx,
-                        float* out) {
+__global__ void k_sobol(SamplerTables tab, uint64_t n, const uint32_t* dims, const uint64_t* idx, float* out) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = sobol_sample(mat, idx[i], dims[i]);
+  const uint32_t c = dims[i];
+  uint4 a[1];
+  sobol_words<1>(tab.nib, idx[i], c & ~3u, a);
+  out[i] = sobol_float((c & 3u) == 0u ? a[0].x : ((c & 3u) == 1u ? a[0].y : ((c & 3u) == 2u ? a[0].z : a[0].w)));
 }
 
 __global__ void k_halton(SamplerTables tab, uint64_t n, const uint32_t* dims, const uint64_t* idx, float* out) {
@@ -2505,12 +2520,11 @@ struct gyt_context {
   Queues q = {};
   uint32_t* d_counter = nullptr;
   uint32_t* h_counter = nullptr;
-  uint32_t* d_sobol = nullptr;
-  uint32_t* d_sobol_bits = nullptr;
+  uint32_t* d_nib = nullptr;  // Sobol' columns combined four index bits at a time (SamplerTables)
   uint16_t* d_hperm = nullptr;  // Halton digit-block tables (halton_tables)
   uint4* d_hdesc = nullptr;
-  uint64_t* d_vdc = nullptr;
-  uint64_t* d_vdc_inv = nullptr;
+  uint64_t* d_enum_fwd = nullptr;
+  uint64_t* d_enum_inv = nullptr;
   double* d_film = nullptr;
   size_t film_bytes = 0;
   float* d_rgb = nullptr;
@@ -2588,7 +2602,7 @@ cudaError_t after_legacy_stream(gyt_context* ctx) {
 }
 
 SamplerTables tables(const gyt_context* c) {
-  return SamplerTables{c->d_sobol, c->d_vdc, c->d_vdc_inv, c->d_sobol_bits, c->d_hperm, c->d_hdesc};
+  return SamplerTables{c->d_nib, c->d_enum_fwd, c->d_enum_inv, c->d_hperm, c->d_hdesc};
 }
 
 Params make_params(const GytRenderParams* p) {
@@ -2626,6 +2640,37 @@ void raster_to_world(const GytCamera& c, double m[16]) {
       for (int k = 0; k < 4; ++k) s += c2w[i][k] * r2c[k][j];
       m[4 * i + j] = s;
     }
+}
+
+// The Sobol' generator columns and the enumeration matrices combined four
+// bits at a time (SamplerTables): entry v of a chunk is the XOR of the chunk's
+// columns over the bits of v.
+void sobol_tables(std::vector<uint32_t>* nib, std::vector<uint64_t>* efwd, std::vector<uint64_t>* einv) {
+  const size_t flat = (size_t)GYT_SOBOL_DIMS * GYT_SOBOL_COLS;
+  nib->assign((size_t)kNibChunks * 16 * kSobolRow, 0u);
+  for (int j = 0; j < kNibChunks; ++j) {
+    uint32_t* chunk = nib->data() + (size_t)j * 16 * kSobolRow;
+    for (int v = 1; v < 16; ++v) {
+      const int top = v >= 8 ? 3 : (v >= 4 ? 2 : (v >= 2 ? 1 : 0));
+      const uint32_t* rest = chunk + (v - (1 << top)) * kSobolRow;
+      for (size_t d = 0; d < (size_t)kSobolRow; ++d) {
+        // column b of dimension d, the matrices read as one array
+        const size_t at = d * GYT_SOBOL_COLS + 4 * j + top;
+        chunk[v * kSobolRow + d] = rest[d] ^ (at < flat ? gyt_sobol_matrices[at] : 0u);
+      }
+    }
+  }
+  auto combine = [](const uint64_t (*rows)[GYT_SOBOL_COLS], std::vector<uint64_t>* out) {
+    out->assign((size_t)GYT_ENUM_M * kEnumChunks * 16, 0ull);
+    for (size_t k = 0; k < (size_t)GYT_ENUM_M * kEnumChunks; ++k) {
+      const uint64_t* col = rows[k / kEnumChunks] + 4 * (k % kEnumChunks);
+      for (int v = 0; v < 16; ++v)
+        for (int b = 0; b < 4; ++b)
+          if (v >> b & 1) (*out)[16 * k + v] ^= col[b];
+    }
+  };
+  combine(gyt_vdc_sobol, efwd);
+  combine(gyt_vdc_sobol_inv, einv);
 }
 
 // Digit-block tables of HaltonSampler with Faure permutations
@@ -2675,7 +2720,7 @@ void halton_tables(std::vector<uint16_t>* perm_out, std::vector<uint4>* desc_out
     const float scale = (float)(0x1.fffffcp-1 / (double)Bn);
     uint32_t bits;
     std::memcpy(&bits, &scale, 4);
-    (*desc_out)[d] = make_uint4((uint32_t)perm_out->size(), (uint32_t)B, n, bits);
+    (*desc_out)[d] = make_uint4((uint32_t)perm_out->size() | (n << 24), (uint32_t)B, (uint32_t)((1ull << 32) / B), bits);
     for (uint32_t i = 0; i < B; ++i) {
       uint32_t r = 0, q = i;
       for (uint32_t j = 0; j < k; ++j, q /= b) r = r * b + fp[b][q % b];
@@ -2891,6 +2936,8 @@ int32_t run_volume(gyt_context* ctx, const gyt_scene* scene, const GytCamera* ca
   const bool equi = (params->flags & GYT_VOLUME_EQUI_ANGULAR) != 0;
   const int g_ext = ctx->pgrid[pindex(kPExtend, W, false)];
   const int g_walk = std::max(1, ctx->sms) * 4;  // grid-stride walks over the queues
+  auto* const vshade = prm.sampler ? (equi ? k_vshade<1, true> : k_vshade<1, false>)
+                                   : (equi ? k_vshade<0, true> : k_vshade<0, false>);
   const Queues q = ctx->q;
   const DebugOut dbg{L_out, cursor_out, nullptr, nullptr, nullptr};
   cudaStream_t sm = ctx->stream;
@@ -2913,14 +2960,12 @@ int32_t run_volume(gyt_context* ctx, const gyt_scene* scene, const GytCamera* ca
     active += n_new;
     if (W == 8) {
       k_extend<8, false><<<g_ext, kBlock, 0, sm>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-      if (equi) k_vshade<8, true><<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
-      else k_vshade<8, false><<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
+      vshade<<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
       k_vshadow<8><<<g_walk, kBlock, 0, sm>>>(P, D, q);
       k_vmis<8><<<g_walk, kBlock, 0, sm>>>(P, D, q);
     } else {
       k_extend<2, false><<<g_ext, kBlock, 0, sm>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-      if (equi) k_vshade<2, true><<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
-      else k_vshade<2, false><<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
+      vshade<<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
       k_vshadow<2><<<g_walk, kBlock, 0, sm>>>(P, D, q);
       k_vmis<2><<<g_walk, kBlock, 0, sm>>>(P, D, q);
     }
@@ -3208,34 +3253,22 @@ int32_t gyt_context_create(int32_t device, gyt_context** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_counter, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_counter, 8 * sizeof(uint32_t));
-  const size_t sob = GYT_SOBOL_DIMS * GYT_SOBOL_COLS;
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_sobol, (sob + 64) * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_sobol, 0, (sob + 64) * sizeof(uint32_t), c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_sobol, gyt_sobol_matrices, sob * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) {
-    // transposed copy: row b = column b of every dimension (see sobol10)
-    std::vector<uint32_t> tr((size_t)64 * kSobolRow, 0u);
-    for (int b = 0; b < 64; ++b)
-      for (int dm = 0; dm < kSobolRow; ++dm) {
-        size_t flat = (size_t)dm * 52 + b;
-        tr[(size_t)b * kSobolRow + dm] = flat < sob ? gyt_sobol_matrices[flat] : 0u;
-      }
-    e = cudaMalloc((void**)&c->d_sobol_bits, tr.size() * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_sobol_bits, tr.data(), tr.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
-  }
+  std::vector<uint32_t> nib;
+  std::vector<uint64_t> efwd, einv;
+  sobol_tables(&nib, &efwd, &einv);
+  auto table = [&](auto** dst, const auto& v) {
+    const size_t bytes = v.size() * sizeof(v[0]);
+    if (e == cudaSuccess) e = cudaMalloc((void**)dst, bytes);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(*dst, v.data(), bytes, cudaMemcpyHostToDevice, c->stream);
+  };
+  table(&c->d_nib, nib);
+  table(&c->d_enum_fwd, efwd);
+  table(&c->d_enum_inv, einv);
   std::vector<uint16_t> hperm;
   std::vector<uint4> hdesc;
   halton_tables(&hperm, &hdesc);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_hperm, hperm.size() * sizeof(uint16_t));
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(c->d_hperm, hperm.data(), hperm.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_hdesc, hdesc.size() * sizeof(uint4));
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(c->d_hdesc, hdesc.data(), hdesc.size() * sizeof(uint4), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_vdc, sizeof(gyt_vdc_sobol));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_vdc, gyt_vdc_sobol, sizeof(gyt_vdc_sobol), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_vdc_inv, sizeof(gyt_vdc_sobol_inv));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_vdc_inv, gyt_vdc_sobol_inv, sizeof(gyt_vdc_sobol_inv), cudaMemcpyHostToDevice, c->stream);
+  table(&c->d_hperm, hperm);
+  table(&c->d_hdesc, hdesc);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming);
@@ -3287,12 +3320,11 @@ void gyt_context_destroy(gyt_context* c) {
   for (void* p : c->adj_allocs) cudaFree(p);
   cudaFree(c->d_counter);
   cudaFreeHost(c->h_counter);
-  cudaFree(c->d_sobol);
-  cudaFree(c->d_sobol_bits);
+  cudaFree(c->d_nib);
   cudaFree(c->d_hperm);
   cudaFree(c->d_hdesc);
-  cudaFree(c->d_vdc);
-  cudaFree(c->d_vdc_inv);
+  cudaFree(c->d_enum_fwd);
+  cudaFree(c->d_enum_inv);
   cudaFree(c->d_film);
   cudaFree(c->d_rgb);
   if (c->bexec) cudaGraphExecDestroy(c->bexec);
@@ -4308,7 +4340,7 @@ int32_t gyt_sobol(gyt_context* ctx, uint64_t n, const uint32_t* dims, const uint
   GYT_CK(ctx, dalloc(tmp, &dout, n));
   GYT_CK(ctx, cudaMemcpyAsync(dd, dims, n * 4, cudaMemcpyHostToDevice, ctx->stream));
   GYT_CK(ctx, cudaMemcpyAsync(di, indices, n * 8, cudaMemcpyHostToDevice, ctx->stream));
-  k_sobol<<<grid_for(n), kBlock, 0, ctx->stream>>>(ctx->d_sobol, n, dd, di, dout);
+  k_sobol<<<grid_for(n), kBlock, 0, ctx->stream>>>(tables(ctx), n, dd, di, dout);
   GYT_CK(ctx, cudaGetLastError());
   GYT_CK(ctx, cudaStreamSynchronize(ctx->stream));
   GYT_CK(ctx, cudaMemcpy(out, dout, n * 4, cudaMemcpyDeviceToHost));
