@@ -27,7 +27,42 @@ GYT_HD float3 cross(float3 a, float3 b) {
 }
 GYT_HD float length(float3 a) { return sqrtf(dot(a, a)); }
 // Vector::Norm divides by the length (math/Linagl.h:527-531)
-GYT_HD float3 norm(float3 a) { return a / length(a); }
+GYT_HD float3 norm_in(float3 a) { return a / length(a); }
+// The same, out of line on the device: a bounce normalises about twenty
+// vectors, the shade kernels are bound by instruction fetch (every warp walks
+// 130 KB of code about once), and a called copy stays in the instruction cache.
+// Its three quotients share y = RN(1 / s): q = RN(a y), then one correction
+// q - RN(q s - a) y rounds as a / s does. Markstein (1990): with y correctly
+// rounded that holds unless a / s lies within 1.5 * 2^-24 ulp of a rounding
+// boundary; all such pairs of 24-bit significands (17.4M, from m s + d = 0 mod
+// 2^24 for |d| <= 3) were checked to round correctly as well. Lengths outside
+// [2^-60, 2^60] divide plainly; a component below 2^-100, whose residual may be
+// subnormal, can be off by one ulp of its own. The sign of the residual keeps
+// that of a zero component. Mesh at 16 spp, shade launches of a render: 16.5
+// ms inlined with nine-operation divisions, 14.9 ms called.
+#ifdef __CUDA_ARCH__
+__device__ __noinline__ float3 norm_plain(float x, float y, float z, float s) { return mk(x / s, y / s, z / s); }
+__device__ __noinline__ float3 norm_call(float x, float y, float z) {
+  const float s = length(mk(x, y, z));  // bounds every component
+  if (!(s < 1.152921504606847e18f && s > 8.673617379884035e-19f)) return norm_plain(x, y, z, s);
+  const float r = __frcp_rn(s);
+  const float qx = __fmul_rn(x, r), qy = __fmul_rn(y, r), qz = __fmul_rn(z, r);
+  return mk(__fmaf_rn(-__fmaf_rn(qx, s, -x), r, qx), __fmaf_rn(-__fmaf_rn(qy, s, -y), r, qy),
+            __fmaf_rn(-__fmaf_rn(qz, s, -z), r, qz));
+}
+#endif
+GYT_HD float3 norm(float3 a) {
+#ifdef __CUDA_ARCH__
+  return norm_call(a.x, a.y, a.z);
+#else
+  return norm_in(a);
+#endif
+}
+// Where a caller's own arithmetic contracts with the normalisation's (its
+// fused multiply-adds then round differently out of line) it takes the inlined
+// one, so that results stay as they are.
+template <bool IN>
+GYT_HD float3 norm_t(float3 a) { return IN ? norm_in(a) : norm(a); }
 GYT_HD float3 vabs(float3 a) { return mk(fabsf(a.x), fabsf(a.y), fabsf(a.z)); }
 GYT_HD bool is_zero(float3 a) { return a.x == 0.f && a.y == 0.f && a.z == 0.f; }
 GYT_HD float comp(float3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }
@@ -417,31 +452,33 @@ struct Hit {
 
 // Sphere::Intersect hit record (shape/Sphere.h:70-117, with the written-back
 // record) under the identity ObjectToWorld (math/Transform.h:296-308).
+template <bool IN = false>
 GYT_D void sphere_hit(float4 s, const Ray& r, float th, Hit* h) {
   float3 c = f3(s);
   float3 hit = r.o + r.d * th;
   float3 sd = (hit - c) * s.w / length(hit - c);
   hit = c + sd;
-  float3 n = norm(hit - c);
+  float3 n = norm_t<IN>(hit - c);
   float3 nl = dot(n, r.d) < 0.f ? n : n * -1.f;
   float3 perr = vabs(c) * gammaf(1) + vabs(sd) * gammaf(6);
   float3 ph = hit - c;
   const float phimax = 2.f * kPi;
   float3 dpdu = mk(-phimax * ph.z, 0.f, phimax * ph.x);
-  float3 su = norm(dpdu - n * dot(n, dpdu));
-  float3 sv = norm(cross(n, su));
+  float3 su = norm_t<IN>(dpdu - n * dot(n, dpdu));
+  float3 sv = norm_t<IN>(cross(n, su));
   h->pos = hit;
   h->perr = perr * (gammaf(3) + 1.f) + vabs(hit) * gammaf(3);
-  h->n = norm(n);
-  h->abs_n = norm(nl);
-  h->wo = norm(r.d * -1.f);
-  h->geo_n = norm(n);
-  h->su = norm(su);
-  h->sv = norm(sv);
+  h->n = norm_t<IN>(n);
+  h->abs_n = norm_t<IN>(nl);
+  h->wo = norm_t<IN>(r.d * -1.f);
+  h->geo_n = norm_t<IN>(n);
+  h->su = norm_t<IN>(su);
+  h->sv = norm_t<IN>(sv);
 }
 
 // Triangle::QueryIntersectionInfo (shape/Triangle.cpp:6-69) and the hit
 // position of Triangle::Intersect (:97).
+template <bool IN = false>
 GYT_D void tri_hit(float3 p0, float3 p1, float3 p2, float3 n0, float3 n1, float3 n2, float3 face, float b1,
                    float b2, float3 ro, float3 rd, Hit* h) {
   float b0 = 1.f - b1 - b2;
@@ -449,15 +486,15 @@ GYT_D void tri_hit(float3 p0, float3 p1, float3 p2, float3 n0, float3 n1, float3
   float xs = fabsf(b0 * p0.x) + fabsf(b1 * p1.x) + fabsf(b2 * p2.x);
   float ys = fabsf(b0 * p0.y) + fabsf(b1 * p1.y) + fabsf(b2 * p2.y);
   float zs = fabsf(b0 * p0.z) + fabsf(b1 * p1.z) + fabsf(b2 * p2.z);
-  float3 ns = norm(n0 * b0 + n1 * b1 + n2 * b2);
+  float3 ns = norm_t<IN>(n0 * b0 + n1 * b1 + n2 * b2);
   h->geo_n = dot(face, ns) < 0.f ? -face : face;
   h->abs_n = dot(h->geo_n, rd) < 0.f ? h->geo_n : h->geo_n * -1.f;
   h->wo = -rd;
   h->perr = mk(xs, ys, zs) * gammaf(7);
   float s = dot(ro - p0, ns) > 0.f ? 1.f : -1.f;
-  float3 du = norm(p1 - p0);
-  float3 dv = norm(cross(ns * s, du));
-  du = norm(cross(dv, ns));
+  float3 du = norm_t<IN>(p1 - p0);
+  float3 dv = norm_t<IN>(cross(ns * s, du));
+  du = norm_t<IN>(cross(dv, ns));
   h->n = ns;
   h->su = du;
   h->sv = dv;
@@ -466,9 +503,10 @@ GYT_D void tri_hit(float3 p0, float3 p1, float3 p2, float3 n0, float3 n1, float3
 // OffsetRayOrigin (math/GeometryUtils.h:39-64): the offset distance
 // d = |n| . pErr, then the origin moved by d along n (towards w) and rounded
 // one float away. A shading kernel that spawns several rays from one point
-// computes d once (offset_dist) and calls offset_origin_d.
+// computes d once (offset_dist) and calls offset_origin_d (out of line, as
+// norm_call).
 GYT_D float offset_dist(float3 perr, float3 n) { return dot(vabs(n), perr); }
-GYT_D float3 offset_origin_d(float3 p, float d, float3 n, float3 w) {
+__device__ __noinline__ float3 offset_origin_d(float3 p, float d, float3 n, float3 w) {
   float3 off = n * d;
   if (dot(w, n) < 0.f) off = -off;
   float3 po = p + off;
@@ -511,11 +549,15 @@ GYT_D float fr_cond1(float c2, float s2, float eta, float k, float cosI) {
   return 0.5f * (Rp + Rs);
 }
 
-// FrConductor with etai = 1 (bsdf/BSDF.cpp:29-51)
+// FrConductor with etai = 1 (bsdf/BSDF.cpp:29-51). Channels of equal eta and k
+// (a grey metal, the reference's default) have equal values: two divisions
+// and two roots instead of six each.
 GYT_D float3 fr_conductor(float cosI, float3 eta, float3 k) {
   cosI = fminf(fmaxf(cosI, -1.f), 1.f);
   float c2 = cosI * cosI, s2 = 1.f - c2;
-  return mk(fr_cond1(c2, s2, eta.x, k.x, cosI), fr_cond1(c2, s2, eta.y, k.y, cosI), fr_cond1(c2, s2, eta.z, k.z, cosI));
+  const float r = fr_cond1(c2, s2, eta.x, k.x, cosI);
+  if (eta.y == eta.x && eta.z == eta.x && k.y == k.x && k.z == k.x) return mk(r, r, r);
+  return mk(r, fr_cond1(c2, s2, eta.y, k.y, cosI), fr_cond1(c2, s2, eta.z, k.z, cosI));
 }
 
 // GGXDistribution with visible-normal sampling (visual/Microfacet.cpp:232-379)
@@ -531,8 +573,9 @@ struct GGX {
     return res;
   }
   GYT_D float project(float3 v) const {
+    if (ax == ay) return ax;
     float inv = 1.f / fmaxf(0.f, 1.f - v.z * v.z);
-    if (ax == ay || inv <= 0.f) return ax;
+    if (inv <= 0.f) return ax;
     float c = v.x * v.x * inv, s = v.y * v.y * inv;
     return sqrtf(c * ax * ax + s * ay * ay);
   }
@@ -615,7 +658,7 @@ struct Lobe {
       float co = wo.z, ci = wi.z;
       if (ci == 0.f || co == 0.f) return mk(0.f, 0.f, 0.f);
       float e = wo.z > 0.f ? eta : 1.f / eta;
-      float3 wh = -norm(wo + wi * e);
+      float3 wh = -norm_in(wo + wi * e);
       wh = wh * sgnf(wh.z);
       float F = fr_dielectric(dot(wo, wh), 1.f, eta);
       float sd = dot(wo, wh) + e * dot(wi, wh);
@@ -644,7 +687,7 @@ struct Lobe {
         dwh = 1.f / (4.f * dot(wi, wh));
       } else {
         float e = wo.z > 0.f ? eta : 1.f / eta;
-        wh = -norm(wo + wi * e);
+        wh = -norm_in(wo + wi * e);
         float sd = dot(wo, wh) + e * dot(wi, wh);
         dwh = fabsf((e * e * dot(wi, wh)) / (sd * sd));
       }
@@ -654,6 +697,75 @@ struct Lobe {
       return p * (refl ? F : (1.f - F));
     }
     return 0.f;
+  }
+
+  // The direction alone of BxDF::Sample (bsdf/BSDF.cpp:80). The MIS half of
+  // direct lighting needs a sample's value and pdf only where its direction
+  // meets the sampled light, which few do (0.5% of the shadow rays' number on
+  // the mesh workload).
+  struct Dir {
+    float3 wi, wh;  // the direction; the GGX half vector
+    float F;        // Fresnel reflectance (glass and GGX dielectric)
+    bool refl;      // reflected (not transmitted)
+    bool ok;        // false: the sample is void (value and pdf 0)
+  };
+
+  GYT_D Dir sample_dir(float3 wo, float u0, float u1, float u2) const {
+    Dir r;
+    r.wi = r.wh = mk(0.f, 0.f, 0.f);
+    r.F = 0.f;
+    r.refl = r.ok = true;
+    if (type == 0) {  // DiffuseBSDF::Sample + CosineSampleHemisphere (visual/Sampling.cpp:5-36)
+      float ox = 2.f * u0 - 1.f, oy = 2.f * u1 - 1.f;
+      float dx = 0.f, dy = 0.f;
+      if (!(ox == 0.f && oy == 0.f)) {
+        float th, rr;
+        if (fabsf(ox) > fabsf(oy)) { rr = ox; th = kPiOver4 * (oy / ox); }
+        else { rr = oy; th = kPiOver2 - kPiOver4 * (ox / oy); }
+        float s, c;
+        sincosf(th, &s, &c);
+        dx = rr * c;
+        dy = rr * s;
+      }
+      float z = sqrtf(fmaxf(0.f, 1.f - dx * dx - dy * dy));
+      r.wi = mk(dx, dy, z);
+      if (wo.z < 0.f) r.wi.z *= -1.f;
+      return r;
+    }
+    if (type == 1) {  // SpecularBSDF::Sample (BSDF.h:200-206)
+      r.wi = mk(-wo.x, -wo.y, wo.z);
+      return r;
+    }
+    if (type == 2) {  // TransmissionBSDF::Sample (BSDF.h:239-268)
+      r.F = fr_dielectric(wo.z, eta1, eta);
+      r.refl = u1 < r.F;
+      if (r.refl) {
+        r.wi = mk(-wo.x, -wo.y, wo.z);
+        return r;
+      }
+      bool entering = wo.z > 0.f;
+      float eI = entering ? eta1 : eta, eT = entering ? eta : eta1;
+      float3 nf = wo.z > 0.f ? mk(0.f, 0.f, 1.f) : mk(0.f, 0.f, -1.f);
+      r.ok = refract(wo, nf, eI / eT, &r.wi);
+      return r;
+    }
+    // MicrofacetReflectionBSDF::Sample (BSDF.h:331-346), RoughDielectricBSDF::Sample (BSDF.h:545-613)
+    r.ok = false;
+    if (wo.z == 0.f || type > 4) return r;
+    r.wh = g.sample(wo * sgnf(wo.z), u0, u1);
+    if (type == 4) {
+      r.F = fr_dielectric(dot(wo, r.wh), 1.f, eta);
+      r.refl = u2 < r.F;
+    }
+    if (r.refl) {
+      r.wi = reflect(wo, r.wh);
+      r.ok = wo.z * r.wi.z > 0.f;
+      return r;
+    }
+    float er = wo.z > 0.f ? 1.f / eta : eta;
+    float3 ff = dot(r.wh, wo) < 0.f ? -r.wh : r.wh;  // Faceforward (GeometryUtils.h:66-68)
+    r.ok = refract(wo, ff, er, &r.wi) && !(wo.z * r.wi.z >= 0.f);
+    return r;
   }
 
   // BxDF::Sample with *pdf starting at 0 (bsdf/BSDF.cpp:80)
@@ -777,9 +889,14 @@ struct Bsdf {
     if ((refl && (f & kRefl)) || (!refl && (f & kTrans))) return lobe.eval(local(wo), local(wi));
     return mk(0.f, 0.f, 0.f);
   }
-  // Not inlined: the shading kernel samples the BSDF twice (the MIS half of
-  // direct lighting and the continuation), and one out-of-line copy keeps its
-  // instruction footprint small (it is instruction-bound).
+  // Not inlined: the shading kernels sample the BSDF at two or three places,
+  // and one out-of-line copy keeps their instruction footprint small (they are
+  // bound by instruction fetch).
+  __device__ __noinline__ bool sample_dir(float3 wo, float3* wi, float u0, float u1, float u2) const {
+    const Lobe::Dir r = lobe.sample_dir(local(wo), u0, u1, u2);
+    *wi = world(r.wi);
+    return r.ok;
+  }
   __device__ __noinline__ float3 sample(float3 wo, float3* wi, float* pdf, float u0, float u1, float u2) const {
     float3 wl;
     float3 f = lobe.sample(local(wo), &wl, pdf, u0, u1, u2);
@@ -872,13 +989,13 @@ GYT_D float env_sin_theta(const EnvDev& e, float v) {  // SinTheta (EnvMap.h:119
 
 GYT_D float3 env_lookup(const EnvDev& e, float3 d) {  // Lookup (EnvMap.h:30-51)
   float u, v;
-  env_dir_to_uv(norm(d), &u, &v);
+  env_dir_to_uv(norm_in(d), &u, &v);
   return env_radiance(e, u, v);
 }
 
 GYT_D float env_pdf_dir(const EnvDev& e, float3 d) {  // PdfDir (EnvMap.h:53-61)
   float u, v;
-  env_dir_to_uv(norm(d), &u, &v);
+  env_dir_to_uv(norm_in(d), &u, &v);
   float st = env_sin_theta(e, v);
   if (st == 0.f) return 0.f;
   int iu = min(max((int)(u * e.w), 0), e.w - 1), iv = min(max((int)(v * e.h), 0), e.h - 1);

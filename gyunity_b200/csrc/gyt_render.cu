@@ -182,11 +182,11 @@ constexpr int shadow_blocks_per_sm() { return 4; }
 template <int W>
 constexpr int extend_blocks_per_sm() { return 5; }
 // The shade kernels, once their blocks are sorted by lobe type, are bound by
-// latency at two blocks per SM (124 registers): a cap of 80 registers (three
-// blocks, some spilled values) shades 11-13% faster on the procedural mesh
-// and the uneven batch, and 64 registers (four blocks) another 3% (2% of the
-// whole render on both). 128-thread blocks at the same occupancy were slower:
-// the sort window is the block.
+// instruction fetch and latency: 64 registers (four blocks of 256, some
+// spilled values) shade the mesh in 13.9 ms a render, 80 registers (three
+// blocks) in 0.9 ms more, 48 (five) in 1.5 more. The block is also what keeps
+// eight warps on the same code: warps that sort a window of their own and run
+// on independently, with every warp slot of the SM filled, took 20% longer.
 constexpr int kShadeBlocksPerSm = 4;
 
 // meta bit 20: the bounce queued an MIS ray whose contribution k_finish adds
@@ -711,10 +711,11 @@ __global__ void __launch_bounds__(kBlock, extend_blocks_per_sm<W>())
 
 // Append to a compact queue: one atomicAdd per warp.
 GYT_D uint32_t queue_slot(uint32_t* count) {
-  cg::coalesced_group g = cg::coalesced_threads();
+  const uint32_t act = __activemask(), lane = threadIdx.x & 31u;
+  const int leader = __ffs(act) - 1;
   uint32_t base = 0;
-  if (g.thread_rank() == 0) base = atomicAdd(count, g.size());
-  return g.shfl(base, 0) + g.thread_rank();
+  if ((int)lane == leader) base = atomicAdd(count, (uint32_t)__popc(act));
+  return __shfl_sync(act, base, leader) + __popc(act & ((1u << lane) - 1u));
 }
 
 // Gradient accumulation: lanes with the same key sum their values first
@@ -858,14 +859,15 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
     float u10[10];
     rng.peek<10>(tab, SAMPLER < 0 ? prm.sampler : (uint32_t)SAMPLER, u10);
     const bool emit = (depth == 0 || delta) && light >= 0;
-    // the continuation's four dimensions (arguments again in right-to-left
-    // order) wait in shared memory while direct lighting runs: four registers
-    // fewer live across it in the 64-register build (blocks of kBlock threads)
-    __shared__ float s_cont[4][kBlock];
-    s_cont[0][threadIdx.x] = emit ? u10[0] : u10[6];
-    s_cont[1][threadIdx.x] = emit ? u10[1] : u10[7];
-    s_cont[2][threadIdx.x] = emit ? u10[2] : u10[8];
-    s_cont[3][threadIdx.x] = emit ? u10[3] : u10[9];
+    // the two BSDF samples' numbers (arguments again in right-to-left order:
+    // z, y, x; rows 0-2 the MIS half, 3-5 the continuation, 6 roulette) wait in
+    // shared memory: seven registers fewer live across the light sample in the
+    // 64-register build (blocks of kBlock threads)
+    __shared__ float s_u[7][kBlock];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s_u[k][threadIdx.x] = u10[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s_u[3 + k][threadIdx.x] = emit ? u10[k] : u10[6 + k];
     if (emit) {
       LightTri l = load_light(s, light);
       if (dot(h.n, h.wo) > 0.f) {
@@ -873,7 +875,6 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
         if (ADJ) grad_emitter(G, s, light, adj * (tp * l.Le));
       }
     } else {
-      float vz = u10[0], vy = u10[1], vx = u10[2];
       float uy = u10[3], ux = u10[4];
       float ul = u10[5];
       rng.cursor += 6;
@@ -894,21 +895,23 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
           lerr = (vabs(l.p0 * bb0) + vabs(l.p1 * bb1) + vabs(l.p2 * bb2)) * gammaf(6);
           labs = l.face;
           pdf = 1.f / l.area;
-          float3 w = h.pos - lpos;
-          if (length(w) == 0.f) {
+          // the direction to the light is that from it, negated (rounding is
+          // symmetric): one normalisation
+          wi = norm(lpos - h.pos);
+          const float3 w = h.pos - lpos;
+          const float w2 = dot(w, w);
+          if (w2 == 0.f) {
             pdf = 0.f;
           } else {
-            w = norm(w);
-            pdf *= dot(h.pos - lpos, h.pos - lpos) / fabsf(dot(ln, -w));
+            pdf *= w2 / fabsf(dot(ln, wi));
             if (isinf(pdf)) pdf = 0.f;
           }
-          wi = norm(lpos - h.pos);
           Li = dot(ln, -wi) > 0.f ? l.Le : mk(0.f, 0.f, 0.f);
         } else {
           // EnvironmentLight::Sample_Li (light/EnvLight.cpp:41-51): a point 2R away
           float3 sd;
           Li = env_sample(s.env, ux, uy, &sd, &pdf);
-          wi = norm(sd);
+          wi = norm_in(sd);
           lpos = h.pos + wi * (2.f * s.env.radius);
           lerr = mk(0.f, 0.f, 0.f);
           labs = wi;
@@ -936,18 +939,29 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
                                     __int_as_float(li), 0.f);
           }
         }
-        // BSDF-sampled half of the MIS estimate (Integrator.cpp:66-101)
+        // BSDF-sampled half of the MIS estimate (Integrator.cpp:66-101): the
+        // direction alone first, and its value and pdf only where it meets
+        // the light triangle (an environment light is met by most)
         float3 wi2;
-        float pdf2;
-        float3 f2 = sbsdf.sample(h.wo, &wi2, &pdf2, vx, vy, vz);
-        if (FROZEN) f2 = refit(f2, wi2);
-        float cos2 = fabsf(dot(h.n, wi2));
-        if (pdf2 != 0.f && !is_zero(f2)) {
+        const float vz = s_u[0][threadIdx.x], vy = s_u[1][threadIdx.x], vx = s_u[2][threadIdx.x];
+        float pdf2 = 0.f;
+        float3 f2 = mk(0.f, 0.f, 0.f);
+        bool ok;
+        if (env_light) {
+          f2 = sbsdf.sample(h.wo, &wi2, &pdf2, vx, vy, vz);
+          ok = pdf2 != 0.f && !is_zero(f2);
+        } else {
+          ok = sbsdf.sample_dir(h.wo, &wi2, vx, vy, vz);
+        }
+        if (ok) {
           float3 o2 = offset_origin_d(h.pos, ofs_d, h.abs_n, wi2) + wi2 * kRayEps;  // SpawnRay
           // the light triangle again from the light table rather than kept live
           // across the BSDF evaluation and sampling
           float lpdf = env_light ? env_pdf_dir(s.env, wi2) : tri_light_pdf(load_light(s, li), h, o2, wi2);
-          if (lpdf != 0.f) {
+          if (lpdf != 0.f && !env_light) f2 = sbsdf.sample(h.wo, &wi2, &pdf2, vx, vy, vz);
+          if (FROZEN) f2 = refit(f2, wi2);
+          if (lpdf != 0.f && pdf2 != 0.f && !is_zero(f2)) {
+            float cos2 = fabsf(dot(h.n, wi2));
             float w2 = power_heuristic(pdf2, lpdf);
             float3 c = tp * (f2 * cos2 / pdf2) * w2 / lsel;
             const uint32_t j = queue_slot(q.counts + 1);
@@ -963,8 +977,8 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
       }
     }
     // continuation (PT.cpp:45-62)
-    float rz = s_cont[0][threadIdx.x], ry = s_cont[1][threadIdx.x], rx = s_cont[2][threadIdx.x];
-    const float urr = s_cont[3][threadIdx.x];
+    float rz = s_u[3][threadIdx.x], ry = s_u[4][threadIdx.x], rx = s_u[5][threadIdx.x];
+    const float urr = s_u[6][threadIdx.x];
     rng.cursor += 3;
     float3 wi;
     float pdf;
@@ -1746,7 +1760,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_light_trace(DevScene s, LtCam c, 
       } else {
         const int k = prim - s.n_tris;
         Ray r = sphere_object_ray(o, d, __int_as_float(0x7f800000), 0.f);
-        sphere_hit(__ldg(s.spheres + k), r, tmax, &h);
+        sphere_hit<true>(__ldg(s.spheres + k), r, tmax, &h);
         mat = __ldg(s.sphere_mat + k);
       }
       Bsdf bsdf;
@@ -1964,15 +1978,15 @@ GYT_D void vpt_direct_queue(const DevScene& s, const Queues& q, const VPoint& p,
     // AreaLight::Sample_Li -> Shape::Sample(ref) -> Triangle::Sample
     const LightPoint lp = light_point(l, ux, uy);
     float pdf = 1.f / l.area;
-    float3 w = p.pos - lp.pos;
-    if (length(w) == 0.f) {
+    const float3 wi = norm(lp.pos - p.pos);  // as shade_path
+    const float3 w = p.pos - lp.pos;
+    const float w2 = dot(w, w);
+    if (w2 == 0.f) {
       pdf = 0.f;
     } else {
-      w = norm(w);
-      pdf *= dot(p.pos - lp.pos, p.pos - lp.pos) / fabsf(dot(lp.n, -w));
+      pdf *= w2 / fabsf(dot(lp.n, wi));
       if (isinf(pdf)) pdf = 0.f;
     }
-    const float3 wi = norm(lp.pos - p.pos);
     const float3 Li = dot(lp.n, -wi) > 0.f ? l.Le : mk(0.f, 0.f, 0.f);
     if (pdf > 0.f && !is_zero(Li)) {
       float spdf, cos_t = 1.f;
@@ -1995,14 +2009,14 @@ GYT_D void vpt_direct_queue(const DevScene& s, const Queues& q, const VPoint& p,
   float3 wi, f;
   float pdf, cos_t = 1.f;
   if (p.surface) {
-    f = bsdf->sample(p.wo, &wi, &pdf, vx, vy, vz);
-    cos_t = fabsf(dot(p.n, wi));
+    // the direction first (as shade_path)
+    if (!bsdf->sample_dir(p.wo, &wi, vx, vy, vz)) return;
   } else {
     const float ph = phase_sample(g, p.wo, vx, vy, &wi);
     f = mk(ph, ph, ph);
     pdf = ph;
   }
-  if (pdf != 0.f && !is_zero(f)) {
+  if (p.surface || pdf != 0.f) {
     // Intersection::SpawnRay (visual/Intersection.h:74-78)
     const float3 o2 = offset_origin(p.pos, p.perr, p.abs_n, wi) + wi * kRayEps;
     Hit hh;
@@ -2011,7 +2025,11 @@ GYT_D void vpt_direct_queue(const DevScene& s, const Queues& q, const VPoint& p,
     hh.abs_n = p.abs_n;
     hh.n = p.n;
     const float lpdf = tri_light_pdf(l, hh, o2, wi);
-    if (lpdf != 0.f) {
+    if (lpdf != 0.f && p.surface) {
+      f = bsdf->sample(p.wo, &wi, &pdf, vx, vy, vz);
+      cos_t = fabsf(dot(p.n, wi));
+    }
+    if (lpdf != 0.f && pdf != 0.f && !is_zero(f)) {
       const float w2 = power_heuristic(pdf, lpdf);
       const float3 c = tp * (f * cos_t / pdf * w2 / lsel);
       const uint32_t j = queue_slot(q.counts + 1);
