@@ -363,9 +363,14 @@ __device__ __noinline__ bool wt_intersect_fp64(const WtRay& r, float3 p0, float3
 // weights of p1 (b1) and p2 (b2), the convention of Triangle::Intersect
 // (shape/Triangle.cpp:71-103). Accepts 0 <= t <= tmax. With SETTLE (segment
 // rays: shadow rays) a distance within 2e-6 relative of tmax is settled in FP64.
-template <bool SETTLE = false>
+// dir: the ray's direction where the caller's r does not hold it (called
+// before the FP64 test only).
+struct KeepDir {
+  GYT_D void operator()(float3*) const {}
+};
+template <bool SETTLE = false, class Dir = KeepDir>
 GYT_D bool wt_intersect(const WtRay& r, float3 p0, float3 p1, float3 p2, float tmax, float* t, float* b1,
-                        float* b2) {
+                        float* b2, Dir dir = Dir{}) {
   float3 A = p0 - r.o, B = p1 - r.o, C = p2 - r.o;
   float Akz = comp(A, r.kz), Bkz = comp(B, r.kz), Ckz = comp(C, r.kz);
   float Ax = comp(A, r.kx) - r.Sx * Akz, Ay = comp(A, r.ky) - r.Sy * Akz;
@@ -392,7 +397,9 @@ GYT_D bool wt_intersect(const WtRay& r, float3 p0, float3 p1, float3 p2, float t
   if (SETTLE) {
     if (!(th >= 0.f && th <= tmax * 1.000002f)) return false;
     if (th >= tmax * 0.999998f) {
-      if (!wt_intersect_fp64(r, p0, p1, p2, tmax)) return false;
+      WtRay rd = r;
+      dir(&rd.d);
+      if (!wt_intersect_fp64(rd, p0, p1, p2, tmax)) return false;
       th = fminf(th, tmax);
     }
   } else if (!(th >= 0.f && th <= tmax)) {
