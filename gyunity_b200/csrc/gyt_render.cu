@@ -119,6 +119,22 @@ struct GradOut {
 };
 constexpr uint32_t kPendValid = 1u << 31;
 
+// The number of live paths of a wavefront iteration: known to the host, or
+// left on the device by the iteration before (see wavefront_loop).
+struct Live {
+  const uint32_t* prev;  // null: n
+  uint32_t n;
+  GYT_D uint32_t get() const { return prev ? *(const volatile uint32_t*)prev : n; }
+};
+
+// Every kernel of a wavefront iteration may be launched while the one before
+// it still runs (launch_next): it lets the next one start and waits for the
+// one before to end before it touches memory.
+GYT_D void chain_start() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 struct Params {
   uint32_t spp, max_depth, rr_depth;
   uint32_t sampler;  // 0 Sobol', 1 Halton (GYT_SAMPLER_HALTON)
@@ -907,6 +923,7 @@ GYT_D void gen_path(PathBuf& dst, uint32_t k, uint32_t x, uint32_t y, uint32_t s
 __global__ void __launch_bounds__(kBlock) k_generate(PathBuf dst, uint32_t base, uint32_t n_new,
                                                      unsigned long long first, Cam cam, uint32_t spp,
                                                      const uint32_t* __restrict__ list, SamplerTables tab) {
+  chain_start();
   uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n_new) return;
   unsigned long long p = first + j;
@@ -924,8 +941,10 @@ __global__ void __launch_bounds__(kBlock) k_generate(PathBuf dst, uint32_t base,
 
 template <int W, bool COUNT>
 __global__ void __launch_bounds__(kBlock, extend_blocks_per_sm<W>())
-    k_extend(PathBuf cur, uint32_t n, DevScene s, float4* __restrict__ hits, uint32_t* __restrict__ fetch,
+    k_extend(PathBuf cur, Live live, DevScene s, float4* __restrict__ hits, uint32_t* __restrict__ fetch,
              unsigned long long* counters) {
+  chain_start();
+  const uint32_t n = live.get();
   persistent_trace<W, false, COUNT, false, true>(
       s, fetch, n,
       [&](uint32_t i, float3& o, float3& d, float& tmax, TraceGeo&) {
@@ -1273,8 +1292,11 @@ GYT_D uint32_t coherent_slot(uint32_t i, uint32_t key) {
 
 template <bool FROZEN, int SAMPLER>
 __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
-    k_shade(PathBuf cur, uint32_t n, DevScene s, Params prm, Queues q, SamplerTables tab, DebugOut dbg) {
+    k_shade(PathBuf cur, Live live, DevScene s, Params prm, Queues q, SamplerTables tab, DebugOut dbg) {
+  chain_start();
+  const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
   const uint32_t j = coherent_slot(i, i < n ? shade_class(s, q, i) : kClassIdle);
   if (j != ~0u) shade_path<false, true, FROZEN, SAMPLER>(cur, j, s, prm, q, tab, dbg);
 }
@@ -1337,6 +1359,7 @@ template <int W, bool COUNT>
 __global__ void __launch_bounds__(kBlock, shadow_blocks_per_sm<W>()) k_connect(PathBuf cur, DevScene s, Queues q,
                                                                                 DebugOut dbg,
                                                                                 unsigned long long* counters) {
+  chain_start();
   const uint32_t ns = *(volatile uint32_t*)q.counts;
   persistent_trace<W, true, COUNT>(
       s, q.counts + 3, ns,
@@ -1409,9 +1432,11 @@ GYT_D void film_add(double* film, uint32_t w, uint32_t x, uint32_t y, float3 L) 
 
 // Finished paths go to the film (FP64 atomics, Film::AddSample with the box
 // filter, visual/Film.h:61-87); live paths are compacted into the next pool.
-__global__ void __launch_bounds__(kBlock) k_finish(PathBuf cur, PathBuf nxt, uint32_t n, double* __restrict__ film,
+__global__ void __launch_bounds__(kBlock) k_finish(PathBuf cur, PathBuf nxt, Live live, double* __restrict__ film,
                                                    uint32_t res_x, uint32_t* __restrict__ counter,
                                                    const float4* __restrict__ madd, DebugOut dbg) {
+  chain_start();
+  const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
   uint32_t meta = i < n ? cur.meta[i] : 0u;
@@ -1468,6 +1493,7 @@ __global__ void __launch_bounds__(kBlock) k_generate_adj(PathBuf dst, AdjBuf A, 
                                                          unsigned long long first, Cam cam, uint32_t spp,
                                                          const uint32_t* __restrict__ list, SamplerTables tab,
                                                          AdjIn in) {
+  chain_start();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n_new) return;
   const unsigned long long p = first + j;
@@ -1509,8 +1535,10 @@ __global__ void __launch_bounds__(kBlock) k_generate_adj(PathBuf dst, AdjBuf A, 
   A.pend[k] = make_uint2(0u, 0u);
 }
 
-__global__ void __launch_bounds__(kBlock) k_shade_adj(PathBuf cur, AdjBuf A, uint32_t n, DevScene s, Params prm,
+__global__ void __launch_bounds__(kBlock) k_shade_adj(PathBuf cur, AdjBuf A, Live live, DevScene s, Params prm,
                                                       Queues q, SamplerTables tab, GradOut G) {
+  chain_start();
+  const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   shade_path<true>(cur, i, s, prm, q, tab, DebugOut{}, A, G);
@@ -1518,6 +1546,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_adj(PathBuf cur, AdjBuf A, uin
 
 template <int W>
 __global__ void __launch_bounds__(kBlock, shadow_blocks_per_sm<W>()) k_shadow_adj(PathBuf cur, AdjBuf A, DevScene s, Queues q, GradOut G) {
+  chain_start();
   const uint32_t n = *(volatile uint32_t*)q.counts;
   persistent_trace<W, true, false>(
       s, q.counts + 3, n,
@@ -1543,6 +1572,7 @@ __global__ void __launch_bounds__(kBlock, shadow_blocks_per_sm<W>()) k_shadow_ad
 
 template <int W>
 __global__ void __launch_bounds__(kBlock) k_mis_adj(PathBuf cur, AdjBuf A, DevScene s, Queues q, GradOut G) {
+  chain_start();
   const uint32_t n = *(volatile uint32_t*)(q.counts + 1);
   persistent_trace<W, false, false>(
       s, q.counts + 4, n,
@@ -1559,8 +1589,10 @@ __global__ void __launch_bounds__(kBlock) k_mis_adj(PathBuf cur, AdjBuf A, DevSc
 
 // Live paths (and their adjoint state) compacted; finished paths are done
 // (their gradient was moved at their last bounce).
-__global__ void __launch_bounds__(kBlock) k_finish_adj(PathBuf cur, PathBuf nxt, AdjBuf A, AdjBuf AN, uint32_t n,
+__global__ void __launch_bounds__(kBlock) k_finish_adj(PathBuf cur, PathBuf nxt, AdjBuf A, AdjBuf AN, Live live,
                                                        uint32_t* __restrict__ counter) {
+  chain_start();
+  const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
   const uint32_t meta = i < n ? cur.meta[i] : 0u;
@@ -2277,8 +2309,10 @@ GYT_D void vpt_direct_queue(const DevScene& s, const Queues& q, const VPoint& p,
 // shadow segment. The light point is recomputed from its two numbers where it
 // is used rather than kept.
 template <int SAMPLER, bool EQUI>
-__global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, uint32_t n, DevScene s, Params prm,
+__global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, Live live, DevScene s, Params prm,
                                                                  Queues q, SamplerTables tab) {
+  chain_start();
+  const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 h4 = q.hit[i];
@@ -2473,6 +2507,7 @@ __global__ void __launch_bounds__(kBlock, EQUI ? 4 : 3) k_vshade(PathBuf cur, ui
 // tracer's occlusion test settles it. Grid-stride over the queue.
 template <int W>
 __global__ void __launch_bounds__(kBlock) k_vshadow(PathBuf cur, DevScene s, Queues q) {
+  chain_start();
   const uint32_t nq = *(volatile uint32_t*)q.counts;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nq; j += gridDim.x * blockDim.x) {
     const float4 a = q.so[j], b = q.sd[j], c4 = q.sc[j], x = q.madd[j];
@@ -2532,6 +2567,7 @@ __global__ void __launch_bounds__(kBlock) k_vshadow(PathBuf cur, DevScene s, Que
 // emission and the transmittance (Integrator.cpp:86-101). Grid-stride.
 template <int W>
 __global__ void __launch_bounds__(kBlock) k_vmis(PathBuf cur, DevScene s, Queues q) {
+  chain_start();
   const uint32_t nq = *(volatile uint32_t*)(q.counts + 1);
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nq; j += gridDim.x * blockDim.x) {
     const float4 a = q.mo[j], b = q.md[j], c4 = q.mc[j];
@@ -3148,10 +3184,95 @@ int32_t run_light_tracing(gyt_context* ctx, const gyt_scene* scene, const GytCam
   return GYT_OK;
 }
 
-// VolPathTracing (n == 0: every sample of the render into d_film; else the
-// listed (x, y, s) samples, radiance and dimensions used out).
 int32_t ensure_pool(gyt_context* ctx);
 unsigned long long wavefront_bound(unsigned long long total, uint32_t max_depth, uint32_t pool);
+
+// Launches a kernel of kBlock threads a block that starts with chain_start()
+// behind the kernel before it on the stream: its blocks may become resident
+// while that one drains, which hides the launch.
+template <class... P, class... A>
+cudaError_t launch_next(cudaStream_t s, uint32_t grid, void (*k)(P...), A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(kBlock);
+  c.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+
+// Blocks of a persistent kernel with one lane per ray at least.
+inline uint32_t trace_grid(int full, uint32_t n) { return std::min((uint32_t)full, std::max(1u, grid_for(n))); }
+
+// Iterations launched between two waits of the host, and the live paths up to
+// which they are: an iteration's grid is sized for the first one's count, so
+// the blocks past the live paths, which end at once, cost more as that grows.
+// A 64x64 render at 4 spp takes 650 us with a wait per iteration, 423 with
+// chains of 4, 408 with 8 (442 without overlapped launches); 1M paths 1820,
+// 1758 and 1752. From 2M paths an iteration takes milliseconds and the wait
+// does not show.
+constexpr uint32_t kChain = 8;
+constexpr uint32_t kChainPaths = 1u << 20;
+
+struct LoopStats {
+  unsigned long long slots = 0;
+  uint32_t iterations = 0, launches = 0;
+};
+
+// The wavefront loop of every render: refills the pool (generate) and runs an
+// iteration (iterate) until all paths have ended; `life` bounds a path's
+// iterations. While paths remain to be generated the host reads the live
+// count after every iteration. Once none remain and at most kChainPaths are
+// live, up to kChain iterations follow each other without it: each takes its
+// count from the device and has counters of its own, and the host waits once
+// for all of them.
+template <class Generate, class Iterate, class Counts>
+int32_t wavefront_loop(gyt_context* ctx, unsigned long long total, uint32_t life, unsigned long long max_iters,
+                       bool single, const char* what, Generate generate, Iterate iterate, Counts on_counts,
+                       LoopStats* out) {
+  cudaStream_t s = ctx->stream;
+  unsigned long long generated = 0;
+  uint32_t active = 0, age = 0;
+  int cur = 0;
+  while (generated < total || active > 0) {
+    const uint32_t n_new = (uint32_t)std::min<unsigned long long>(ctx->capacity - active, total - generated);
+    if (n_new) age = 0;
+    uint32_t chain = 1;
+    if (!single && generated + n_new == total && active + n_new <= kChainPaths)
+      chain = std::min(kChain, std::max(1u, life > age ? life - age : 1u));
+    GYT_CK(ctx, cudaMemsetAsync(ctx->q.counts, 0, (size_t)chain * 8 * sizeof(uint32_t), s));
+    if (n_new) {
+      GYT_CK(ctx, generate(cur, active, n_new, generated));
+      ++out->launches;
+    }
+    generated += n_new;
+    active += n_new;
+    for (uint32_t k = 0; k < chain; ++k, cur ^= 1) {
+      Queues q = ctx->q;
+      q.counts = ctx->q.counts + 8 * k;
+      GYT_CK(ctx, iterate(cur, Live{k ? q.counts - 3 : nullptr, active}, active, q, &out->launches));
+    }
+    GYT_CK(ctx, cudaMemcpyAsync(ctx->h_counter, ctx->q.counts, (size_t)chain * 8 * sizeof(uint32_t),
+                                cudaMemcpyDeviceToHost, s));
+    GYT_CK(ctx, cudaStreamSynchronize(s));
+    for (uint32_t k = 0; k < chain && active > 0; ++k) {
+      const uint32_t* h = ctx->h_counter + 8 * k;
+      on_counts(active, h, n_new);
+      out->slots += active;
+      ++out->iterations;
+      ++age;
+      active = h[5];
+    }
+    if (out->iterations > max_iters) return fail(ctx, GYT_ERR_WATCHDOG, std::string(what) + ": wavefront iteration cap reached");
+  }
+  return GYT_OK;
+}
+
+// VolPathTracing (n == 0: every sample of the render into d_film; else the
+// listed (x, y, s) samples, radiance and dimensions used out).
 
 int32_t run_volume(gyt_context* ctx, const gyt_scene* scene, const GytCamera* camera, const GytRenderParams* params,
                    uint64_t n, const uint32_t* xys, double* d_film, float* L_out, uint32_t* cursor_out,
@@ -3181,53 +3302,35 @@ int32_t run_volume(gyt_context* ctx, const gyt_scene* scene, const GytCamera* ca
   const int g_walk = std::max(1, ctx->sms) * 4;  // grid-stride walks over the queues
   auto* const vshade = prm.sampler ? (equi ? k_vshade<1, true> : k_vshade<1, false>)
                                    : (equi ? k_vshade<0, true> : k_vshade<0, false>);
-  const Queues q = ctx->q;
   const DebugOut dbg{L_out, cursor_out, nullptr, nullptr, nullptr};
   cudaStream_t sm = ctx->stream;
   // a crossing of a material-less surface takes a wavefront iteration without a bounce
-  const unsigned long long max_iters = wavefront_bound(count, params->max_depth + 65, ctx->capacity);
-  unsigned long long generated = 0;
-  uint32_t active = 0, iters = 0, launches = 0;
-  unsigned long long slots = 0;
-  int cur = 0;
+  const uint32_t life = params->max_depth + 65;
+  LoopStats ls;
   GYT_CK(ctx, cudaEventRecord(ctx->ev0, sm));
-  while (generated < count || active > 0) {
-    const uint32_t n_new = (uint32_t)std::min<unsigned long long>(ctx->capacity - active, count - generated);
-    GYT_CK(ctx, cudaMemsetAsync(q.counts, 0, 8 * sizeof(uint32_t), sm));
+  auto generate = [&](int cur, uint32_t base, uint32_t n_new, unsigned long long first) {
+    return launch_next(sm, grid_for(n_new), k_generate, ctx->pool[cur], base, n_new, first, cam, params->spp, xys, tab);
+  };
+  auto iterate = [&](int cur, Live live, uint32_t bound, const Queues& q, uint32_t* launches) {
     const PathBuf P = ctx->pool[cur], N = ctx->pool[cur ^ 1];
-    if (n_new) {
-      k_generate<<<grid_for(n_new), kBlock, 0, sm>>>(P, active, n_new, generated, cam, params->spp, xys, tab);
-      ++launches;
-    }
-    generated += n_new;
-    active += n_new;
-    if (W == 8) {
-      k_extend<8, false><<<g_ext, kBlock, 0, sm>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-      vshade<<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
-      k_vshadow<8><<<g_walk, kBlock, 0, sm>>>(P, D, q);
-      k_vmis<8><<<g_walk, kBlock, 0, sm>>>(P, D, q);
-    } else {
-      k_extend<2, false><<<g_ext, kBlock, 0, sm>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-      vshade<<<grid_for(active), kBlock, 0, sm>>>(P, active, D, prm, q, tab);
-      k_vshadow<2><<<g_walk, kBlock, 0, sm>>>(P, D, q);
-      k_vmis<2><<<g_walk, kBlock, 0, sm>>>(P, D, q);
-    }
-    k_finish<<<grid_for(active), kBlock, 0, sm>>>(P, N, active, d_film, cam.res_x, q.counts + 5, q.madd, dbg);
-    launches += 5;
-    GYT_CK(ctx, cudaGetLastError());
-    GYT_CK(ctx, cudaMemcpyAsync(ctx->h_counter, q.counts, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, sm));
-    GYT_CK(ctx, cudaStreamSynchronize(sm));
-    slots += active;
-    active = ctx->h_counter[5];
-    cur ^= 1;
-    if (++iters > max_iters) return fail(ctx, GYT_ERR_WATCHDOG, "render_volume: wavefront iteration cap reached");
-  }
+    const uint32_t g = trace_grid(g_ext, bound), gw = trace_grid(g_walk, bound);
+    *launches += 5;
+    launch_next(sm, g, W == 8 ? k_extend<8, false> : k_extend<2, false>, P, live, D, q.hit, q.counts + 2, nullptr);
+    launch_next(sm, grid_for(bound), vshade, P, live, D, prm, q, tab);
+    launch_next(sm, gw, W == 8 ? k_vshadow<8> : k_vshadow<2>, P, D, q);
+    launch_next(sm, gw, W == 8 ? k_vmis<8> : k_vmis<2>, P, D, q);
+    launch_next(sm, grid_for(bound), k_finish, P, N, live, d_film, cam.res_x, q.counts + 5, q.madd, dbg);
+    return cudaGetLastError();
+  };
+  st = wavefront_loop(ctx, count, life, wavefront_bound(count, life, ctx->capacity), false, "render_volume", generate,
+                      iterate, [](uint32_t, const uint32_t*, uint32_t) {}, &ls);
+  if (st) return st;
   GYT_CK(ctx, cudaEventRecord(ctx->ev1, sm));
   GYT_CK(ctx, cudaEventSynchronize(ctx->ev1));
   if (stats) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    *stats = GytRenderStats{count, slots, iters, launches, ms};
+    *stats = GytRenderStats{count, ls.slots, ls.iterations, ls.launches, ms};
   }
   return GYT_OK;
 }
@@ -3269,7 +3372,7 @@ int32_t ensure_pool(gyt_context* ctx) {
   GYT_CK(ctx, dalloc(L, &q.mc, n));
   GYT_CK(ctx, dalloc(L, &q.hit, n));
   GYT_CK(ctx, dalloc(L, &q.madd, n));
-  GYT_CK(ctx, dalloc(L, &q.counts, 8));
+  GYT_CK(ctx, dalloc(L, &q.counts, 8 * kChain));
   ctx->pool_cap = ctx->capacity;
   return ensure_adj_reset(ctx);
 }
@@ -3311,85 +3414,63 @@ int32_t run_paths(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, cons
   Params prm = make_params(p);
   SamplerTables tab = tables(ctx);
   cudaStream_t s = ctx->stream;
-  unsigned long long generated = 0;
-  uint32_t active = 0, iters = 0;
-  unsigned long long rays = 0;
-  int cur = 0;
   const bool prof = ctx->profile > 0, cnt = ctx->profile > 1;
-  uint32_t launches = 0;
-  unsigned long long slots = 0;
-  const int W = scene->dev.wnodes ? 8 : 2;
+  const DevScene& D = scene->dev;
+  const int W = D.wnodes ? 8 : 2;
   const int g_ext = ctx->pgrid[pindex(kPExtend, W, cnt)], g_sh = ctx->pgrid[pindex(kPShadow, W, cnt)];
-  Queues q = ctx->q;
+  unsigned long long* const C = cnt ? ctx->d_counters : nullptr;
+  auto* const extend = W == 8 ? (cnt ? k_extend<8, true> : k_extend<8, false>)
+                              : (cnt ? k_extend<2, true> : k_extend<2, false>);
+  auto* const connect = W == 8 ? (cnt ? k_connect<8, true> : k_connect<8, false>)
+                               : (cnt ? k_connect<2, true> : k_connect<2, false>);
+  auto* const shade = D.sparams ? (prm.sampler ? k_shade<true, 1> : k_shade<true, 0>)
+                                : (prm.sampler ? k_shade<false, 1> : k_shade<false, 0>);
   if (cnt) GYT_CK(ctx, cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), s));
-  uint32_t hcounts[8];
+  LoopStats ls;
   GYT_CK(ctx, after_legacy_stream(ctx));
   GYT_CK(ctx, cudaEventRecord(ctx->ev0, s));
-  while (generated < total || active > 0) {
-    uint32_t n_new = (uint32_t)std::min<unsigned long long>(ctx->capacity - active, total - generated);
-    GYT_CK(ctx, cudaMemsetAsync(q.counts, 0, 8 * sizeof(uint32_t), s));
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[0], s));
-    if (n_new) {
-      k_generate<<<grid_for(n_new), kBlock, 0, s>>>(ctx->pool[cur], active, n_new, generated, cam, p->spp, d_list, tab);
-      ++launches;
-    }
-    generated += n_new;
-    active += n_new;
+  auto mark = [&](int k) {
+    if (prof) cudaEventRecord(ctx->kev[k], s);
+  };
+  bool marked = false;  // the iteration's start, by generate
+  auto generate = [&](int cur, uint32_t base, uint32_t n_new, unsigned long long first) {
+    mark(0);
+    marked = true;
+    return launch_next(s, grid_for(n_new), k_generate, ctx->pool[cur], base, n_new, first, cam, p->spp, d_list, tab);
+  };
+  auto iterate = [&](int cur, Live live, uint32_t bound, const Queues& q, uint32_t* launches) {
     const PathBuf P = ctx->pool[cur], N = ctx->pool[cur ^ 1];
-    const DevScene& D = scene->dev;
-    unsigned long long* C = ctx->d_counters;
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[1], s));
-    if (W == 8) {
-      if (cnt) k_extend<8, true><<<g_ext, kBlock, 0, s>>>(P, active, D, q.hit, q.counts + 2, C);
-      else k_extend<8, false><<<g_ext, kBlock, 0, s>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-    } else {
-      if (cnt) k_extend<2, true><<<g_ext, kBlock, 0, s>>>(P, active, D, q.hit, q.counts + 2, C);
-      else k_extend<2, false><<<g_ext, kBlock, 0, s>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-    }
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[2], s));
-    if (D.sparams) {
-      if (prm.sampler) k_shade<true, 1><<<grid_for(active), kBlock, 0, s>>>(P, active, D, prm, q, tab, dbg);
-      else k_shade<true, 0><<<grid_for(active), kBlock, 0, s>>>(P, active, D, prm, q, tab, dbg);
-    } else {
-      if (prm.sampler) k_shade<false, 1><<<grid_for(active), kBlock, 0, s>>>(P, active, D, prm, q, tab, dbg);
-      else k_shade<false, 0><<<grid_for(active), kBlock, 0, s>>>(P, active, D, prm, q, tab, dbg);
-    }
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[3], s));
+    if (!marked) mark(0);
+    marked = false;
+    mark(1);
+    launch_next(s, trace_grid(g_ext, bound), extend, P, live, D, q.hit, q.counts + 2, C);
+    mark(2);
+    launch_next(s, grid_for(bound), shade, P, live, D, prm, q, tab, dbg);
+    mark(3);
     // shadow and MIS rays in one launch (profile slot 3; slot 4 stays empty)
-    if (W == 8) {
-      if (cnt) k_connect<8, true><<<g_sh, kBlock, 0, s>>>(P, D, q, dbg, C + 2);
-      else k_connect<8, false><<<g_sh, kBlock, 0, s>>>(P, D, q, dbg, nullptr);
-    } else {
-      if (cnt) k_connect<2, true><<<g_sh, kBlock, 0, s>>>(P, D, q, dbg, C + 2);
-      else k_connect<2, false><<<g_sh, kBlock, 0, s>>>(P, D, q, dbg, nullptr);
+    launch_next(s, trace_grid(g_sh, bound), connect, P, D, q, dbg, C ? C + 2 : nullptr);
+    mark(4);
+    mark(5);
+    launch_next(s, grid_for(bound), k_finish, P, N, live, d_film, cam.res_x, q.counts + 5, q.madd, dbg);
+    mark(6);
+    *launches += 4;
+    return cudaGetLastError();
+  };
+  auto on_counts = [&](uint32_t n, const uint32_t* h, uint32_t n_new) {
+    if (!prof) return;
+    for (int k = 0; k < 6; ++k) {
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, ctx->kev[k], ctx->kev[k + 1]);
+      ctx->prof.ms[k] += ms;
+      if ((k != 0 || n_new) && k != 4) ctx->prof.launches[k]++;
     }
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[4], s));
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[5], s));
-    k_finish<<<grid_for(active), kBlock, 0, s>>>(P, N, active, d_film, cam.res_x, q.counts + 5, q.madd, dbg);
-    if (prof) GYT_CK(ctx, cudaEventRecord(ctx->kev[6], s));
-    launches += 4;
-    GYT_CK(ctx, cudaGetLastError());
-    GYT_CK(ctx, cudaMemcpyAsync(ctx->h_counter, q.counts, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GYT_CK(ctx, cudaStreamSynchronize(s));
-    std::memcpy(hcounts, ctx->h_counter, sizeof(hcounts));
-    if (prof) {
-      for (int k = 0; k < 6; ++k) {
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, ctx->kev[k], ctx->kev[k + 1]);
-        ctx->prof.ms[k] += ms;
-        if ((k != 0 || n_new) && k != 4) ctx->prof.launches[k]++;
-      }
-      ctx->prof.rays[0] += active;
-      ctx->prof.rays[1] += hcounts[0];
-      ctx->prof.rays[2] += hcounts[1];
-    }
-    slots += active;
-    rays += active;
-    active = hcounts[5];
-    cur ^= 1;
-    if (++iters > wavefront_bound(total, p->max_depth, ctx->capacity))
-      return fail(ctx, GYT_ERR_WATCHDOG, "render: wavefront iteration cap reached");
-  }
+    ctx->prof.rays[0] += n;
+    ctx->prof.rays[1] += h[0];
+    ctx->prof.rays[2] += h[1];
+  };
+  st = wavefront_loop(ctx, total, p->max_depth, wavefront_bound(total, p->max_depth, ctx->capacity), prof, "render",
+                      generate, iterate, on_counts, &ls);
+  if (st) return st;
   GYT_CK(ctx, cudaEventRecord(ctx->ev1, s));
   GYT_CK(ctx, cudaEventSynchronize(ctx->ev1));
   if (cnt) {
@@ -3402,9 +3483,9 @@ int32_t run_paths(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, cons
   }
   if (stats) {
     stats->paths = total;
-    stats->path_slots = slots;
-    stats->iterations = iters;
-    stats->launches = launches;
+    stats->path_slots = ls.slots;
+    stats->iterations = ls.iterations;
+    stats->launches = ls.launches;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     stats->ms = ms;
@@ -3431,47 +3512,35 @@ int32_t run_adjoint(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, co
   const int g_ext = ctx->pgrid[pindex(kPExtend, W, false)], g_sh = ctx->pgrid[pindex(kPShadow, W, false)],
             g_mis = ctx->pgrid[pindex(kPMis, W, false)];
   const DevScene& D = scene->dev;
-  const Queues q = ctx->q;
-  unsigned long long generated = 0;
-  uint32_t active = 0, iters = 0, launches = 0;
-  int cur = 0;
+  LoopStats ls;
   GYT_CK(ctx, after_legacy_stream(ctx));
   GYT_CK(ctx, cudaEventRecord(ctx->ev0, s));
-  while (generated < total || active > 0) {
-    const uint32_t n_new = (uint32_t)std::min<unsigned long long>(ctx->capacity - active, total - generated);
-    GYT_CK(ctx, cudaMemsetAsync(q.counts, 0, 8 * sizeof(uint32_t), s));
+  auto generate = [&](int cur, uint32_t base, uint32_t n_new, unsigned long long first) {
+    return launch_next(s, grid_for(n_new), k_generate_adj, ctx->pool[cur], ctx->adj[cur], base, n_new, first, cam, p->spp,
+                       d_list, tab, in);
+  };
+  auto iterate = [&](int cur, Live live, uint32_t bound, const Queues& q, uint32_t* launches) {
     const PathBuf P = ctx->pool[cur], N = ctx->pool[cur ^ 1];
     const AdjBuf A = ctx->adj[cur], AN = ctx->adj[cur ^ 1];
-    if (n_new) {
-      k_generate_adj<<<grid_for(n_new), kBlock, 0, s>>>(P, A, active, n_new, generated, cam, p->spp, d_list, tab, in);
-      ++launches;
-    }
-    generated += n_new;
-    active += n_new;
-    if (W == 8) k_extend<8, false><<<g_ext, kBlock, 0, s>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-    else k_extend<2, false><<<g_ext, kBlock, 0, s>>>(P, active, D, q.hit, q.counts + 2, nullptr);
-    k_shade_adj<<<grid_for(active), kBlock, 0, s>>>(P, A, active, D, prm, q, tab, G);
-    if (W == 8) k_shadow_adj<8><<<g_sh, kBlock, 0, s>>>(P, A, D, q, G);
-    else k_shadow_adj<2><<<g_sh, kBlock, 0, s>>>(P, A, D, q, G);
-    if (W == 8) k_mis_adj<8><<<g_mis, kBlock, 0, s>>>(P, A, D, q, G);
-    else k_mis_adj<2><<<g_mis, kBlock, 0, s>>>(P, A, D, q, G);
-    k_finish_adj<<<grid_for(active), kBlock, 0, s>>>(P, N, A, AN, active, q.counts + 5);
-    launches += 5;
-    GYT_CK(ctx, cudaGetLastError());
-    GYT_CK(ctx, cudaMemcpyAsync(ctx->h_counter, q.counts, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GYT_CK(ctx, cudaStreamSynchronize(s));
-    active = ctx->h_counter[5];
-    cur ^= 1;
-    if (++iters > wavefront_bound(total, p->max_depth, ctx->capacity))
-      return fail(ctx, GYT_ERR_WATCHDOG, "adjoint: wavefront iteration cap reached");
-  }
+    launch_next(s, trace_grid(g_ext, bound), W == 8 ? k_extend<8, false> : k_extend<2, false>, P, live, D, q.hit,
+                q.counts + 2, nullptr);
+    launch_next(s, grid_for(bound), k_shade_adj, P, A, live, D, prm, q, tab, G);
+    launch_next(s, trace_grid(g_sh, bound), W == 8 ? k_shadow_adj<8> : k_shadow_adj<2>, P, A, D, q, G);
+    launch_next(s, trace_grid(g_mis, bound), W == 8 ? k_mis_adj<8> : k_mis_adj<2>, P, A, D, q, G);
+    launch_next(s, grid_for(bound), k_finish_adj, P, N, A, AN, live, q.counts + 5);
+    *launches += 5;
+    return cudaGetLastError();
+  };
+  st = wavefront_loop(ctx, total, p->max_depth, wavefront_bound(total, p->max_depth, ctx->capacity), false, "adjoint",
+                      generate, iterate, [](uint32_t, const uint32_t*, uint32_t) {}, &ls);
+  if (st) return st;
   GYT_CK(ctx, cudaEventRecord(ctx->ev1, s));
   GYT_CK(ctx, cudaEventSynchronize(ctx->ev1));
   if (stats) {
     stats->paths = total;
     stats->path_slots = 0;
-    stats->iterations = iters;
-    stats->launches = launches;
+    stats->iterations = ls.iterations;
+    stats->launches = ls.launches;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     stats->ms = ms;
@@ -3495,7 +3564,7 @@ int32_t gyt_context_create(int32_t device, gyt_context** out) {
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_counter, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_counter, 8 * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_counter, kChain * 8 * sizeof(uint32_t));
   std::vector<uint32_t> nib;
   std::vector<uint64_t> efwd, einv;
   sobol_tables(&nib, &efwd, &einv);
@@ -5281,13 +5350,13 @@ extern "C" int32_t gyt_render_device_noalloc(gyt_context* ctx, const gyt_scene* 
       k_generate<<<grid_for(n_new), kBlock, 0, s>>>(pool[cur], active, n_new, generated, cam, params->spp, nullptr, tab);
     generated += n_new;
     active += n_new;
-    if (W == 8) k_extend<8, false><<<g_ext, kBlock, 0, s>>>(pool[cur], active, D, q.hit, q.counts + 2, nullptr);
-    else k_extend<2, false><<<g_ext, kBlock, 0, s>>>(pool[cur], active, D, q.hit, q.counts + 2, nullptr);
-    if (prm.sampler) k_shade<false, 1><<<grid_for(active), kBlock, 0, s>>>(pool[cur], active, D, prm, q, tab, DebugOut{});
-    else k_shade<false, 0><<<grid_for(active), kBlock, 0, s>>>(pool[cur], active, D, prm, q, tab, DebugOut{});
+    if (W == 8) k_extend<8, false><<<g_ext, kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, q.hit, q.counts + 2, nullptr);
+    else k_extend<2, false><<<g_ext, kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, q.hit, q.counts + 2, nullptr);
+    if (prm.sampler) k_shade<false, 1><<<grid_for(active), kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, prm, q, tab, DebugOut{});
+    else k_shade<false, 0><<<grid_for(active), kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, prm, q, tab, DebugOut{});
     if (W == 8) k_connect<8, false><<<g_sh, kBlock, 0, s>>>(pool[cur], D, q, DebugOut{}, nullptr);
     else k_connect<2, false><<<g_sh, kBlock, 0, s>>>(pool[cur], D, q, DebugOut{}, nullptr);
-    k_finish<<<grid_for(active), kBlock, 0, s>>>(pool[cur], pool[cur ^ 1], active, d_film, cam.res_x, q.counts + 5,
+    k_finish<<<grid_for(active), kBlock, 0, s>>>(pool[cur], pool[cur ^ 1], Live{nullptr, active}, d_film, cam.res_x, q.counts + 5,
                                                 q.madd,
                                                 DebugOut{});
     GYT_CK(ctx, cudaGetLastError());
