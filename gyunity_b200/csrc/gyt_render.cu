@@ -102,6 +102,8 @@ struct Queues {
   float4* madd; // per path slot: its MIS ray's contribution (k_connect; added by k_finish)
   float4* sx;  // adjoint pass, shadow ray: material bits, d log f / d alpha, light bits, -
   float4* mx;  // adjoint pass, MIS ray: material bits, d log f / d alpha, -, -
+  float4* pc;  // adjoint pass, path slot: the last continuation's contribution, material | kPendValid bits
+  float* pa;   // adjoint pass, path slot: its d log f / d alpha
 };
 
 // Adjoint (path replay) state per path slot, ping-ponged with the pool.
@@ -1058,11 +1060,12 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
   if (ADJ) {
     adj = f3(A.delta[i]);
     const uint2 pend = A.pend[i];
-    if (pend.x & kPendValid) {
-      // the previous continuation's BSDF factor scales all radiance after it
-      const float3 after = f3(A.Ltot[i]) - f3(cur.L[i]);
-      grad_material(G, s, pend.x & ~kPendValid, adj * after, __uint_as_float(pend.y));
-    }
+    // the previous continuation's BSDF factor scales all radiance after it
+    // (its gradient: k_grad_adj)
+    float3 Cd = mk(0.f, 0.f, 0.f);
+    if (pend.x & kPendValid) Cd = adj * (f3(A.Ltot[i]) - f3(cur.L[i]));
+    q.pc[i] = make_float4(Cd.x, Cd.y, Cd.z, __uint_as_float(pend.x));
+    q.pa[i] = __uint_as_float(pend.y);
   }
   if (prim < 0) {
     // PT.cpp:18-21: environment emission on the camera ray or after a delta bounce
@@ -1535,21 +1538,28 @@ __global__ void __launch_bounds__(kBlock) k_generate_adj(PathBuf dst, AdjBuf A, 
   A.pend[k] = make_uint2(0u, 0u);
 }
 
-__global__ void __launch_bounds__(kBlock) k_shade_adj(PathBuf cur, AdjBuf A, Live live, DevScene s, Params prm,
-                                                      Queues q, SamplerTables tab, GradOut G) {
+// The adjoint's bounce, its block sorted by class as the primal's and at the
+// same four blocks per SM: 0.40 -> 0.31 ms for 1M paths (116 registers and
+// unsorted, 14 of 32 lanes ran).
+template <int SAMPLER>
+__global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
+    k_shade_adj(PathBuf cur, AdjBuf A, Live live, DevScene s, Params prm, Queues q, SamplerTables tab, GradOut G) {
   chain_start();
   const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  shade_path<true>(cur, i, s, prm, q, tab, DebugOut{}, A, G);
+  if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
+  const uint32_t j = coherent_slot(i, i < n ? shade_class(s, q, i) : kClassIdle);
+  if (j != ~0u) shade_path<true, true, false, SAMPLER>(cur, j, s, prm, q, tab, DebugOut{}, A, G);
 }
 
+// The queued shadow, then MIS rays of the adjoint pass (k_connect). The
+// gradients of the shadow rays that reach their light wait for k_grad_adj.
 template <int W>
-__global__ void __launch_bounds__(kBlock, shadow_blocks_per_sm<W>()) k_shadow_adj(PathBuf cur, AdjBuf A, DevScene s, Queues q, GradOut G) {
+__global__ void __launch_bounds__(kBlock, shadow_blocks_per_sm<W>()) k_connect_adj(PathBuf cur, AdjBuf A, DevScene s, Queues q, GradOut G) {
   chain_start();
-  const uint32_t n = *(volatile uint32_t*)q.counts;
+  const uint32_t ns = *(volatile uint32_t*)q.counts;
   persistent_trace<W, true, false>(
-      s, q.counts + 3, n,
+      s, q.counts + 3, ns,
       [&](uint32_t j, float3& o, float3& d, float& tmax, TraceGeo&) {
         const float4 a = q.so[j], b = q.sd[j];
         o = f3(a);
@@ -1561,47 +1571,146 @@ __global__ void __launch_bounds__(kBlock, shadow_blocks_per_sm<W>()) k_shadow_ad
         const uint32_t slot = __float_as_uint(q.sd[j].w);
         const float4 c = q.sc[j], l = cur.L[slot];
         cur.L[slot] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, 0.f);
-        const float3 Cd = f3(A.delta[slot]) * f3(c);
-        const float4 x = q.sx[j];
-        grad_material(G, s, __float_as_uint(x.x), Cd, x.y);
-        const int li = __float_as_int(x.z);
-        if (li < s.n_area) grad_emitter(G, s, li, Cd);
+        q.sx[j].w = 1.f;
       },
       nullptr);
-}
-
-template <int W>
-__global__ void __launch_bounds__(kBlock) k_mis_adj(PathBuf cur, AdjBuf A, DevScene s, Queues q, GradOut G) {
-  chain_start();
-  const uint32_t n = *(volatile uint32_t*)(q.counts + 1);
+  const uint32_t nm = *(volatile uint32_t*)(q.counts + 1);
   persistent_trace<W, false, false>(
-      s, q.counts + 4, n,
+      s, q.counts + 4, nm,
       [&](uint32_t j, float3& o, float3& d, float& tmax, TraceGeo&) {
         o = f3(q.mo[j]);
         d = f3(q.md[j]);
         tmax = __int_as_float(0x7f800000);
       },
       [&](uint32_t j, int prim, float, float b1, float b2) {
-        mis_done<true>(cur, q, s, j, prim, b1, b2, DebugOut{}, A, G);
+        mis_done<true, true>(cur, q, s, j, prim, b1, b2, DebugOut{}, A, G);
       },
       nullptr);
+}
+
+// The gradients of an iteration's continuations (one record per path slot) and
+// unoccluded shadow rays: sums of delta C per material (and of delta C d log f
+// / d alpha) and per emission row, in FP64. A block takes 256 records at a
+// time; every record joins its rows' lists in shared memory, and the thread
+// that owns a row walks its list into the row's sums, which stay in shared
+// memory until the block's last record. Moved where they arose, by partial
+// warps that summed equal materials and added them with global atomics, they
+// took half of the shadow kernel and a quarter of the shade kernel. n_mat = 0:
+// more rows than fit shared memory, the records are added one warp at a time.
+__global__ void __launch_bounds__(kBlock) k_grad_adj(AdjBuf A, Live live, DevScene s, Queues q, GradOut G, uint32_t n_mat,
+                                                     uint32_t n_em) {
+  extern __shared__ double s_sum[];  // n_mat x 4, n_em x 3, then the list heads and each row's light
+  __shared__ float4 s_rec[kBlock];   // delta C, d log f / d alpha
+  __shared__ int2 s_next[kBlock];
+  chain_start();
+  const uint32_t np = live.get(), n = np + *(volatile uint32_t*)q.counts;
+  double* const em = s_sum + 4 * n_mat;
+  int* const head = (int*)(em + 3 * n_em);
+  int* const light = head + n_mat + n_em;
+  for (uint32_t k = threadIdx.x; k < 4 * n_mat + 3 * n_em; k += kBlock) s_sum[k] = 0.0;
+  for (uint32_t k = threadIdx.x; k < n_mat + 2 * n_em; k += kBlock) head[k] = -1;
+  __syncthreads();
+  for (uint32_t base = blockIdx.x * kBlock; base < n; base += gridDim.x * kBlock) {
+    const uint32_t i = base + threadIdx.x;
+    uint32_t mat = ~0u;
+    int li = -1;
+    float3 Cd = mk(0.f, 0.f, 0.f);
+    float da = 0.f;
+    if (i < np) {
+      const float4 c = q.pc[i];
+      const uint32_t m = __float_as_uint(c.w);
+      if (m & kPendValid) {
+        mat = m & ~kPendValid;
+        Cd = f3(c);
+        da = q.pa[i];
+      }
+    } else if (i < n) {
+      const float4 x = q.sx[i - np];
+      if (x.w != 0.f) {
+        mat = __float_as_uint(x.x);
+        da = x.y;
+        Cd = f3(A.delta[__float_as_uint(q.sd[i - np].w)]) * f3(q.sc[i - np]);
+        if (__float_as_int(x.z) < s.n_area) li = __float_as_int(x.z);
+      }
+    }
+    if (n_mat == 0u) {
+      if (mat != ~0u) grad_material(G, s, mat, Cd, da);
+      if (li >= 0) grad_emitter(G, s, li, Cd);
+      continue;
+    }
+    s_rec[threadIdx.x] = make_float4(Cd.x, Cd.y, Cd.z, da);
+    int2 next = make_int2(-1, -1);
+    if (mat != ~0u) next.x = atomicExch(head + mat, (int)threadIdx.x);
+    if (li >= 0) {
+      const uint32_t row = __float_as_uint(__ldg(s.ltab + kLightRec * li + 6).w);
+      next.y = atomicExch(head + n_mat + row, (int)threadIdx.x);
+      light[row] = li;  // any light of the row: they share its radiance
+    }
+    s_next[threadIdx.x] = next;
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < n_mat + n_em; r += kBlock) {
+      int e = head[r];
+      if (e < 0) continue;
+      head[r] = -1;
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+      for (; e >= 0; e = r < n_mat ? s_next[e].x : s_next[e].y) {
+        const float4 c = s_rec[e];
+        v0 += c.x;
+        v1 += c.y;
+        v2 += c.z;
+        v3 += ((double)c.x + c.y + c.z) * c.w;
+      }
+      double* const o = r < n_mat ? s_sum + 4 * r : em + 3 * (r - n_mat);
+      o[0] += v0;
+      o[1] += v1;
+      o[2] += v2;
+      if (r < n_mat) o[3] += v3;
+    }
+    __syncthreads();
+  }
+  // f is linear in the albedo and in the emission: the sums over their values
+  for (uint32_t m = threadIdx.x; m < n_mat; m += kBlock) {
+    const uint32_t type = __ldg(s.mtypes + m);
+    if (type != 0u && type != 3u) continue;
+    for (int c = 0; c < 4; ++c) {
+      const double v = s_sum[4 * m + c];
+      const float a = c < 3 ? __ldg(s.mparams + 16u * m + c) : 1.f;
+      if (v != 0.0 && a != 0.f) atomicAdd(G.mat + 4 * (size_t)m + c, v / a);
+    }
+  }
+  for (uint32_t r = threadIdx.x; r < n_em; r += kBlock) {
+    if (light[r] < 0) continue;
+    for (int c = 0; c < 3; ++c) {
+      const double v = em[3 * r + c];
+      const float l = __ldg(s.ltab + kLightRec * light[r] + c).w;
+      if (v != 0.0 && l != 0.f) atomicAdd(G.em + 3 * (size_t)r + c, v / l);
+    }
+  }
 }
 
 // Live paths (and their adjoint state) compacted; finished paths are done
 // (their gradient was moved at their last bounce).
 __global__ void __launch_bounds__(kBlock) k_finish_adj(PathBuf cur, PathBuf nxt, AdjBuf A, AdjBuf AN, Live live,
-                                                       uint32_t* __restrict__ counter) {
+                                                       uint32_t* __restrict__ counter,
+                                                       const float4* __restrict__ madd) {
   chain_start();
   const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
-  const uint32_t meta = i < n ? cur.meta[i] : 0u;
+  uint32_t meta = i < n ? cur.meta[i] : 0u;
+  const bool mis = meta & kMisQueued;  // the MIS contribution of this bounce (k_connect_adj)
+  meta &= ~kMisQueued;
   const uint32_t j = block_compact(meta & kAlive, counter);
   if (!(meta & kAlive)) return;
   nxt.o[j] = cur.o[i];
   nxt.d[j] = cur.d[i];
   nxt.tp[j] = cur.tp[i];
-  nxt.L[j] = cur.L[i];
+  float4 L4 = cur.L[i];
+  if (mis) {
+    const float4 m = madd[i];
+    L4 = make_float4(L4.x + m.x, L4.y + m.y, L4.z + m.z, 0.f);
+  }
+  nxt.L[j] = L4;
   nxt.sidx[j] = cur.sidx[i];
   nxt.meta[j] = meta;
   nxt.pix[j] = cur.pix[i];
@@ -2729,14 +2838,14 @@ inline uint32_t grid_for(uint64_t n) { return (uint32_t)((n + kBlock - 1) / kBlo
 
 // Persistent traversal kernels and their grid sizes (blocks per SM at full
 // occupancy times the SM count), computed once per context.
-enum { kPExtend = 0, kPShadow = 1, kPMis = 2 };
-constexpr int kPersistentKinds = 3 * 2 * 2;  // kernel x width (2, 8) x counting
+enum { kPExtend = 0, kPShadow = 1 };
+constexpr int kPersistentKinds = 2 * 2 * 2;  // kernel x width (2, 8) x counting
 inline int pindex(int kind, int w, bool count) { return (kind * 2 + (w == 8 ? 1 : 0)) * 2 + (count ? 1 : 0); }
 
 template <int W, bool C>
 const void* persistent_fn(int kind) {
   if (kind == kPExtend) return (const void*)k_extend<W, C>;
-  return (const void*)k_connect<W, C>;  // shadow and MIS rays (kPMis: grid of the adjoint's MIS kernel)
+  return (const void*)k_connect<W, C>;  // shadow and MIS rays
 }
 
 }  // namespace
@@ -3197,8 +3306,9 @@ unsigned long long wavefront_bound(unsigned long long total, uint32_t max_depth,
 // behind the kernel before it on the stream: its blocks may become resident
 // while that one drains, which hides the launch.
 template <class... P, class... A>
-cudaError_t launch_next(cudaStream_t s, uint32_t grid, void (*k)(P...), A... args) {
+cudaError_t launch_next(cudaStream_t s, uint32_t grid, size_t smem, void (*k)(P...), A... args) {
   cudaLaunchConfig_t c = {};
+  c.dynamicSmemBytes = smem;
   c.gridDim = dim3(grid);
   c.blockDim = dim3(kBlock);
   c.stream = s;
@@ -3208,6 +3318,10 @@ cudaError_t launch_next(cudaStream_t s, uint32_t grid, void (*k)(P...), A... arg
   c.attrs = &at;
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+cudaError_t launch_next(cudaStream_t s, uint32_t grid, void (*k)(P...), A... args) {
+  return launch_next(s, grid, (size_t)0, k, args...);
 }
 
 // Blocks of a persistent kernel with one lane per ray at least.
@@ -3398,6 +3512,8 @@ int32_t ensure_adj(gyt_context* ctx) {
   }
   GYT_CK(ctx, dalloc(L, &ctx->q.sx, n));
   GYT_CK(ctx, dalloc(L, &ctx->q.mx, n));
+  GYT_CK(ctx, dalloc(L, &ctx->q.pc, n));
+  GYT_CK(ctx, dalloc(L, &ctx->q.pa, n));
   ctx->adj_cap = ctx->pool_cap;
   return GYT_OK;
 }
@@ -3515,9 +3631,14 @@ int32_t run_adjoint(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, co
   const SamplerTables tab = tables(ctx);
   cudaStream_t s = ctx->stream;
   const int W = scene->dev.wnodes ? 8 : 2;
-  const int g_ext = ctx->pgrid[pindex(kPExtend, W, false)], g_sh = ctx->pgrid[pindex(kPShadow, W, false)],
-            g_mis = ctx->pgrid[pindex(kPMis, W, false)];
+  const int g_ext = ctx->pgrid[pindex(kPExtend, W, false)], g_sh = ctx->pgrid[pindex(kPShadow, W, false)];
   const DevScene& D = scene->dev;
+  // k_grad_adj's sums and lists, while they leave room for four blocks per SM
+  // (eight blocks per SM in its grid: 4.39 ms a pass of 1M paths, four 4.48,
+  // two 4.91)
+  uint32_t n_mat = scene->n_materials, n_em = scene->n_emission;
+  size_t grad_smem = (size_t)n_mat * (4 * 8 + 4) + (size_t)n_em * (3 * 8 + 8);
+  if (grad_smem > 40960) n_mat = n_em = grad_smem = 0;
   LoopStats ls;
   GYT_CK(ctx, after_legacy_stream(ctx));
   GYT_CK(ctx, cudaEventRecord(ctx->ev0, s));
@@ -3530,10 +3651,10 @@ int32_t run_adjoint(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, co
     const AdjBuf A = ctx->adj[cur], AN = ctx->adj[cur ^ 1];
     launch_next(s, trace_grid(g_ext, bound), W == 8 ? k_extend<8, false> : k_extend<2, false>, P, live, D, q.hit,
                 q.counts + 2, nullptr);
-    launch_next(s, grid_for(bound), k_shade_adj, P, A, live, D, prm, q, tab, G);
-    launch_next(s, trace_grid(g_sh, bound), W == 8 ? k_shadow_adj<8> : k_shadow_adj<2>, P, A, D, q, G);
-    launch_next(s, trace_grid(g_mis, bound), W == 8 ? k_mis_adj<8> : k_mis_adj<2>, P, A, D, q, G);
-    launch_next(s, grid_for(bound), k_finish_adj, P, N, A, AN, live, q.counts + 5);
+    launch_next(s, grid_for(bound), prm.sampler ? k_shade_adj<1> : k_shade_adj<0>, P, A, live, D, prm, q, tab, G);
+    launch_next(s, trace_grid(g_sh, bound), W == 8 ? k_connect_adj<8> : k_connect_adj<2>, P, A, D, q, G);
+    launch_next(s, trace_grid(std::max(1, ctx->sms) * 8, bound), grad_smem, k_grad_adj, A, live, D, q, G, n_mat, n_em);
+    launch_next(s, grid_for(bound), k_finish_adj, P, N, A, AN, live, q.counts + 5, (const float4*)q.madd);
     *launches += 5;
     return cudaGetLastError();
   };
@@ -3609,16 +3730,13 @@ int32_t gyt_context_create(int32_t device, gyt_context** out) {
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     c->sms = sms;
-    for (int kind = 0; kind < 3 && e == cudaSuccess; ++kind)
+    for (int kind = 0; kind < 2 && e == cudaSuccess; ++kind)
       for (int w : {2, 8})
         for (int cntm = 0; cntm < 2 && e == cudaSuccess; ++cntm) {
           const void* fn = w == 8 ? (cntm ? persistent_fn<8, true>(kind) : persistent_fn<8, false>(kind))
                                   : (cntm ? persistent_fn<2, true>(kind) : persistent_fn<2, false>(kind));
           int nb = 0;
           e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kBlock, 0);
-          // MIS rays are rare (only BSDF samples that would reach the sampled
-          // light): one block per SM keeps the launch cheap
-          if (kind == kPMis) nb = 1;
           c->pgrid[pindex(kind, w, cntm != 0)] = std::max(1, nb) * std::max(1, sms);
         }
   }
