@@ -201,7 +201,7 @@ template <int W>
 constexpr int extend_blocks_per_sm() { return 5; }
 // The shade kernels, once their blocks are sorted by lobe type, are bound by
 // instruction fetch and latency: 64 registers (four blocks of 256, some
-// spilled values) shade the mesh in 13.9 ms a render, 80 registers (three
+// spilled values) shade the mesh in 13.5 ms a render, 80 registers (three
 // blocks) in 0.9 ms more, 48 (five) in 1.5 more. The block is also what keeps
 // eight warps on the same code: warps that sort a window of their own and run
 // on independently, with every warp slot of the SM filled, took 20% longer.
@@ -1035,7 +1035,12 @@ GYT_D void grad_emitter(const GradOut& G, const DevScene& s, int li, float3 Cd) 
 // SAMPLER: 0 Sobol', 1 Halton, -1 prm.sampler at run time. A kernel compiled
 // for one sampler keeps fewer registers live than one with both (-2.4% shade
 // time on the uneven batch).
-template <bool ADJ, bool DEFER = false, bool FROZEN = false, int SAMPLER = -1>
+//
+// ENV: false for scenes without an environment light, whose code (25 of the
+// kernel's 130 KB) is then not compiled in: shade launches of a render, mesh
+// 13.98 -> 13.53 ms, batch of 76M paths 46.5 -> 45.0, Cornell box 0.815 ->
+// 0.793.
+template <bool ADJ, bool DEFER, bool FROZEN, int SAMPLER, bool ENV>
 GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const Params& prm, const Queues& q,
                       SamplerTables tab, const DebugOut& dbg, const AdjBuf& A = AdjBuf{}, const GradOut& G = GradOut{}) {
   float4 h4 = q.hit[i];
@@ -1069,7 +1074,7 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
   }
   if (prim < 0) {
     // PT.cpp:18-21: environment emission on the camera ray or after a delta bounce
-    if ((depth == 0 || delta) && s.has_env) add_L(tp * env_lookup(s.env, rd));
+    if (ENV && (depth == 0 || delta) && s.has_env) add_L(tp * env_lookup(s.env, rd));
   } else {
     Hit h;
     uint32_t mat;
@@ -1133,7 +1138,7 @@ GYT_D void shade_path(const PathBuf& cur, uint32_t i, const DevScene& s, const P
       float lsel = 0.f;
       int li = s.n_lights > 0 ? sample_light(s, ul, &lsel) : 0;
       if (lsel > 0.f) {
-        const bool env_light = li >= s.n_area;
+        const bool env_light = ENV && li >= s.n_area;
         LightTri l;
         float3 wi, Li, lpos, lerr, labs;
         float pdf;
@@ -1293,7 +1298,7 @@ GYT_D uint32_t coherent_slot(uint32_t i, uint32_t key) {
   return order[threadIdx.x];
 }
 
-template <bool FROZEN, int SAMPLER>
+template <bool FROZEN, int SAMPLER, bool ENV>
 __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
     k_shade(PathBuf cur, Live live, DevScene s, Params prm, Queues q, SamplerTables tab, DebugOut dbg) {
   chain_start();
@@ -1301,7 +1306,7 @@ __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
   const uint32_t j = coherent_slot(i, i < n ? shade_class(s, q, i) : kClassIdle);
-  if (j != ~0u) shade_path<false, true, FROZEN, SAMPLER>(cur, j, s, prm, q, tab, dbg);
+  if (j != ~0u) shade_path<false, true, FROZEN, SAMPLER, ENV>(cur, j, s, prm, q, tab, dbg);
 }
 
 // MIS-ray result of one queue entry (every MIS kernel). DEFER: the
@@ -1541,7 +1546,7 @@ __global__ void __launch_bounds__(kBlock) k_generate_adj(PathBuf dst, AdjBuf A, 
 // The adjoint's bounce, its block sorted by class as the primal's and at the
 // same four blocks per SM: 0.40 -> 0.31 ms for 1M paths (116 registers and
 // unsorted, 14 of 32 lanes ran).
-template <int SAMPLER>
+template <int SAMPLER, bool ENV>
 __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
     k_shade_adj(PathBuf cur, AdjBuf A, Live live, DevScene s, Params prm, Queues q, SamplerTables tab, GradOut G) {
   chain_start();
@@ -1549,7 +1554,7 @@ __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= n) return;  // the whole block is idle
   const uint32_t j = coherent_slot(i, i < n ? shade_class(s, q, i) : kClassIdle);
-  if (j != ~0u) shade_path<true, true, false, SAMPLER>(cur, j, s, prm, q, tab, DebugOut{}, A, G);
+  if (j != ~0u) shade_path<true, true, false, SAMPLER, ENV>(cur, j, s, prm, q, tab, DebugOut{}, A, G);
 }
 
 // The queued shadow, then MIS rays of the adjoint pass (k_connect). The
@@ -1796,7 +1801,7 @@ __global__ void __launch_bounds__(kBlock, extend_blocks_per_sm<W>())
 // One path per thread over a grid sized for the whole pool (threads past
 // the live count return at once): the work per path varies a lot, and the
 // block scheduler balances it far better than a grid-stride loop does.
-template <int SAMPLER>
+template <int SAMPLER, bool ENV>
 __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
     k_shade_batch(PathBuf cur, const IterState* __restrict__ st, Queues q, SamplerTables tab) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1805,7 +1810,7 @@ __global__ void __launch_bounds__(kBlock, kShadeBlocksPerSm)
   const uint32_t j = coherent_slot(i, i < n ? shade_class(c_insts[cur.inst[i]].s, q, i) : kClassIdle);
   if (j == ~0u) return;
   const Inst& I = c_insts[cur.inst[j]];
-  shade_path<false, true, false, SAMPLER>(cur, j, I.s, I.prm, q, tab, DebugOut{});
+  shade_path<false, true, false, SAMPLER, ENV>(cur, j, I.s, I.prm, q, tab, DebugOut{});
 }
 
 // Shadow then MIS rays of the batch in one launch (k_connect, every ray with
@@ -3549,8 +3554,9 @@ int32_t run_paths(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, cons
                               : (cnt ? k_extend<2, true> : k_extend<2, false>);
   auto* const connect = W == 8 ? (cnt ? k_connect<8, true> : k_connect<8, false>)
                                : (cnt ? k_connect<2, true> : k_connect<2, false>);
-  auto* const shade = D.sparams ? (prm.sampler ? k_shade<true, 1> : k_shade<true, 0>)
-                                : (prm.sampler ? k_shade<false, 1> : k_shade<false, 0>);
+  auto* const shade = D.sparams   ? (prm.sampler ? k_shade<true, 1, true> : k_shade<true, 0, true>)
+                      : D.has_env ? (prm.sampler ? k_shade<false, 1, true> : k_shade<false, 0, true>)
+                                  : (prm.sampler ? k_shade<false, 1, false> : k_shade<false, 0, false>);
   if (cnt) GYT_CK(ctx, cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), s));
   LoopStats ls;
   GYT_CK(ctx, after_legacy_stream(ctx));
@@ -3637,6 +3643,8 @@ int32_t run_adjoint(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, co
   const int W = scene->dev.wnodes ? 8 : 2;
   const int g_ext = ctx->pgrid[pindex(kPExtend, W, false)], g_sh = ctx->pgrid[pindex(kPShadow, W, false)];
   const DevScene& D = scene->dev;
+  auto* const shade = D.has_env ? (prm.sampler ? k_shade_adj<1, true> : k_shade_adj<0, true>)
+                                : (prm.sampler ? k_shade_adj<1, false> : k_shade_adj<0, false>);
   // k_grad_adj's sums and lists, while they leave room for four blocks per SM
   // (eight blocks per SM in its grid: 4.39 ms a pass of 1M paths, four 4.48,
   // two 4.91)
@@ -3655,7 +3663,7 @@ int32_t run_adjoint(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, co
     const AdjBuf A = ctx->adj[cur], AN = ctx->adj[cur ^ 1];
     launch_next(s, trace_grid(g_ext, bound), W == 8 ? k_extend<8, false> : k_extend<2, false>, P, live, D, q.hit,
                 q.counts + 2, nullptr);
-    launch_next(s, grid_for(bound), prm.sampler ? k_shade_adj<1> : k_shade_adj<0>, P, A, live, D, prm, q, tab, G);
+    launch_next(s, grid_for(bound), shade, P, A, live, D, prm, q, tab, G);
     launch_next(s, trace_grid(g_sh, bound), W == 8 ? k_connect_adj<8> : k_connect_adj<2>, P, A, D, q, G);
     launch_next(s, trace_grid(std::max(1, ctx->sms) * 8, bound), grad_smem, k_grad_adj, A, live, D, q, G, n_mat, n_em);
     launch_next(s, grid_for(bound), k_finish_adj, P, N, A, AN, live, q.counts + 5, (const float4*)q.madd);
@@ -4905,13 +4913,15 @@ namespace {
 struct BatchPlan {
   int W = 2;
   int sampler = -1;  // 0 / 1: every instance samples with Sobol' / Halton (the shade kernel compiled for it)
+  bool env = true;   // some instance has an environment light
   uint32_t stride_grid = 0, ext_grid = 0, sh_grid = 0, shade_grid = 0;
 };
 
-BatchPlan batch_plan(const gyt_context* ctx, int W, int sampler) {
+BatchPlan batch_plan(const gyt_context* ctx, int W, int sampler, bool env) {
   BatchPlan b;
   b.W = W;
   b.sampler = sampler;
+  b.env = env;
   const GytBatchConfig& c = ctx->bcfg;
   const int wi = W == 8 ? 1 : 0;
   const uint32_t sms = (uint32_t)std::max(1, ctx->sms);
@@ -4942,9 +4952,10 @@ cudaError_t enqueue_half(gyt_context* ctx, const BatchPlan& b, const PathBuf& P,
   if (b.W == 8) k_extend_batch<8><<<b.ext_grid, kBlock, 0, s>>>(P, st, q.hit, q.counts + 2);
   else k_extend_batch<2><<<b.ext_grid, kBlock, 0, s>>>(P, st, q.hit, q.counts + 2);
   if (ev) cudaEventRecord(ev[2], s);
-  if (b.sampler == 0) k_shade_batch<0><<<b.shade_grid, kBlock, 0, s>>>(P, st, q, tab);
-  else if (b.sampler == 1) k_shade_batch<1><<<b.shade_grid, kBlock, 0, s>>>(P, st, q, tab);
-  else k_shade_batch<-1><<<b.shade_grid, kBlock, 0, s>>>(P, st, q, tab);
+  auto* const shade = b.sampler == 0 ? (b.env ? k_shade_batch<0, true> : k_shade_batch<0, false>)
+                      : b.sampler == 1 ? (b.env ? k_shade_batch<1, true> : k_shade_batch<1, false>)
+                                       : k_shade_batch<-1, true>;
+  shade<<<b.shade_grid, kBlock, 0, s>>>(P, st, q, tab);
   if (ev) cudaEventRecord(ev[3], s);
   if (b.W == 8) k_connect_batch<8><<<b.sh_grid, kBlock, 0, s>>>(P, q);
   else k_connect_batch<2><<<b.sh_grid, kBlock, 0, s>>>(P, q);
@@ -4959,7 +4970,7 @@ constexpr uint32_t kKernelsPerHalf = 7;
 // The batched render as one graph: a while-loop node whose body is two
 // half-iterations (pool 0 -> 1 -> 0); k_batch_end sets the loop condition.
 int32_t ensure_batch_graph(gyt_context* ctx, const BatchPlan& b) {
-  const uint64_t key[6] = {(uint64_t)b.W | ((uint64_t)(b.sampler + 1) << 8), (uint64_t)b.stride_grid,
+  const uint64_t key[6] = {(uint64_t)b.W | ((uint64_t)(b.sampler + 1) << 8) | ((uint64_t)b.env << 16), (uint64_t)b.stride_grid,
                            ((uint64_t)b.ext_grid << 32) | b.sh_grid, (uint64_t)b.shade_grid,
                            (uint64_t)(uintptr_t)ctx->pool[0].o, (uint64_t)ctx->pool_cap};
   if (ctx->bexec && std::memcmp(key, ctx->bkey, sizeof(key)) == 0) return GYT_OK;
@@ -5057,7 +5068,9 @@ int32_t run_batch(gyt_context* ctx, const BatchInput& in, GytRenderStats* stats)
   int sampler = in.insts.empty() ? 0 : (int)in.insts[0].prm.sampler;
   for (const Inst& I : in.insts)
     if ((int)I.prm.sampler != sampler) sampler = -1;
-  const BatchPlan b = batch_plan(ctx, in.W, sampler);
+  bool env = false;
+  for (const Inst& I : in.insts) env = env || I.s.has_env;
+  const BatchPlan b = batch_plan(ctx, in.W, sampler, env);
   std::lock_guard<std::mutex> lock(g_batch_mutex);
   // profiling (gyt_context_set_profile) times every kernel: host loop
   const bool prof = ctx->profile > 0;
@@ -5459,8 +5472,9 @@ extern "C" int32_t gyt_render_device_noalloc(gyt_context* ctx, const gyt_scene* 
     active += n_new;
     if (W == 8) k_extend<8, false><<<g_ext, kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, q.hit, q.counts + 2, nullptr);
     else k_extend<2, false><<<g_ext, kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, q.hit, q.counts + 2, nullptr);
-    if (prm.sampler) k_shade<false, 1><<<grid_for(active), kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, prm, q, tab, DebugOut{});
-    else k_shade<false, 0><<<grid_for(active), kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, prm, q, tab, DebugOut{});
+    auto* const shade = D.has_env ? (prm.sampler ? k_shade<false, 1, true> : k_shade<false, 0, true>)
+                                  : (prm.sampler ? k_shade<false, 1, false> : k_shade<false, 0, false>);
+    shade<<<grid_for(active), kBlock, 0, s>>>(pool[cur], Live{nullptr, active}, D, prm, q, tab, DebugOut{});
     if (W == 8) k_connect<8, false><<<g_sh, kBlock, 0, s>>>(pool[cur], D, q, DebugOut{}, nullptr);
     else k_connect<2, false><<<g_sh, kBlock, 0, s>>>(pool[cur], D, q, DebugOut{}, nullptr);
     k_finish<<<grid_for(active), kBlock, 0, s>>>(pool[cur], pool[cur ^ 1], Live{nullptr, active}, d_film, cam.res_x, q.counts + 5,
