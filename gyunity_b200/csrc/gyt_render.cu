@@ -9,16 +9,15 @@
 //               the MIS next-event estimate (queued as shadow / MIS rays),
 //               continuation BSDF sample, Russian roulette
 //                                                  PT.cpp:16-65, Integrator.cpp:9-107
-//   k_shadow    next-event shadow rays (any hit) from a compact queue
-//                                                  Visibility.cpp:7-10
-//   k_mis       BSDF-sampled MIS rays (closest hit) from a compact queue
-//                                                  Integrator.cpp:86-101
+//   k_connect   next-event shadow rays (any hit), then BSDF-sampled MIS rays
+//               (closest hit), both from compact queues
+//                                                  Visibility.cpp:7-10, Integrator.cpp:86-101
 //   k_finish    film accumulation of finished paths (FP64 atomics) and
-//               compaction of live paths into the other pool (warp-aggregated
-//               atomics)                           Film.h:61-87
-// The three traversal kernels are persistent: lanes whose ray is done fetch
-// the next queue entry before each traversal step (dynamic ray fetching), so
-// warps stay full while rays of very different lengths are in flight.
+//               compaction of live paths into the other pool (one atomic per
+//               block)                             Film.h:61-87
+// The traversal kernels are persistent: lanes whose ray is done fetch the next
+// queue entry (dynamic ray fetching), so warps stay full while rays of very
+// different lengths are in flight.
 // Path state is SoA in HBM; pools are ping-ponged each iteration so live
 // paths stay dense and new paths fill the tail.
 #include <cuda_runtime.h>
