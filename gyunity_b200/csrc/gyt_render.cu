@@ -2905,10 +2905,11 @@ __global__ void k_gather_int(uint32_t n, const int* __restrict__ index, const in
 }
 
 // ------------------------------------------------------------- host side ---
-// Ray queries run through a workspace of fixed size (46 MB, allocated by the
-// first one): 28 bytes in and 16 out per ray.
+// Ray queries run through a workspace of the context, 28 bytes in and 16 out per
+// ray, at most kQueryRays rays (46 MB) at a time. It grows to the largest query,
+// in the 2 MB blocks that device memory comes in.
 constexpr uint64_t kQueryRays = 1u << 20;
-constexpr size_t kQueryBytes = 44;
+constexpr size_t kQueryBytes = 44, kQueryBlock = 2u << 20;
 
 struct gyt_context {
   int device = 0;
@@ -2930,7 +2931,8 @@ struct gyt_context {
   size_t film_bytes = 0;
   float* d_rgb = nullptr;
   size_t rgb_bytes = 0;
-  unsigned char* d_query = nullptr;  // rays and results of gyt_intersect, kQueryRays at a time
+  unsigned char* d_query = nullptr;  // rays and results of gyt_intersect
+  size_t query_bytes = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t ev_in = nullptr;  // orders a render after the caller's legacy-stream work
   std::vector<void*> pool_allocs;
@@ -4720,7 +4722,15 @@ int32_t gyt_intersect(gyt_context* ctx, const gyt_scene* scene, uint64_t n, cons
   if (!ctx || !scene || (n && !rays)) return fail(ctx, GYT_ERR_INVALID, "intersect: null argument");
   if (n == 0) return GYT_OK;
   GYT_CK(ctx, cudaSetDevice(ctx->device));
-  if (!ctx->d_query) GYT_CK(ctx, cudaMalloc((void**)&ctx->d_query, kQueryRays * kQueryBytes));
+  const size_t need = std::min(n, kQueryRays) * kQueryBytes;
+  if (need > ctx->query_bytes) {
+    cudaFree(ctx->d_query);
+    ctx->d_query = nullptr;
+    ctx->query_bytes = 0;
+    const size_t bytes = (need + kQueryBlock - 1) / kQueryBlock * kQueryBlock;
+    GYT_CK(ctx, cudaMalloc((void**)&ctx->d_query, bytes));
+    ctx->query_bytes = bytes;
+  }
   cudaStream_t s = ctx->stream;
   for (uint64_t i = 0; i < n; i += kQueryRays) {
     const uint64_t m = std::min<uint64_t>(kQueryRays, n - i);

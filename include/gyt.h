@@ -210,7 +210,10 @@ int32_t gyt_trace_paths(gyt_context* ctx, const gyt_scene* scene, const GytCamer
  * (host rays: 7 floats each = origin, direction, tmax; tmin = 0). Outputs
  * (host, may be NULL): prim (-1 = miss; for any_hit 1/0), t, b1, b2 where b1
  * and b2 weight vertices 1 and 2 as Triangle::Intersect reports them
- * (shape/Triangle.cpp:71-103). BVHAccel::Intersect (accelerator/BVHAccel.cpp:401-487). */
+ * (shape/Triangle.cpp:71-103). BVHAccel::Intersect (accelerator/BVHAccel.cpp:401-487).
+ * The context keeps the rays and answers of its largest query on the device (44
+ * bytes a ray, at most 2^20 rays) until it is destroyed; larger queries run
+ * through that memory in passes. */
 int32_t gyt_intersect(gyt_context* ctx, const gyt_scene* scene, uint64_t n, const float* rays,
                       int32_t any_hit, int32_t* prim, float* t, float* b1, float* b2);
 
