@@ -4338,9 +4338,11 @@ int32_t gyt_render_device(gyt_context* ctx, const gyt_scene* scene, const GytCam
 }
 
 // The context's FP64 film and RGB staging buffers of the host-image renders and
-// the film outputs (grown to the largest request, kept until the context is
-// destroyed). Allocated and freed by every call they cost 0.1 to 3 ms of it
-// (the fogged box at 512x512: 7.8 ms a call for 6.0 ms of kernels).
+// the film outputs, grown to the largest request. Allocated and freed by every
+// call they cost 0.1 to 3 ms of it (the fogged box at 512x512: 7.8 ms a call
+// for 6.0 ms of kernels). gyt_render and gyt_render_batch keep them until the
+// context is destroyed; the other calls give back (HostFilmBound) what they
+// needed beyond kKeepFilm of each.
 int32_t ensure_host_films(gyt_context* ctx, size_t fb, size_t rb) {
   if (fb > ctx->film_bytes) {
     cudaFree(ctx->d_film);
@@ -4358,6 +4360,29 @@ int32_t ensure_host_films(gyt_context* ctx, size_t fb, size_t rb) {
   }
   return GYT_OK;
 }
+
+// A 2048x2048 film of the volumetric renders, whose kernels then take far
+// longer than the allocations.
+constexpr size_t kKeepFilm = 128u << 20;
+
+// On leaving its scope frees the buffers that the call grew beyond kKeepFilm
+// (the call has waited for its stream, or failed; cudaFree waits as well).
+struct HostFilmBound {
+  gyt_context* ctx;
+  const size_t film = ctx->film_bytes, rgb = ctx->rgb_bytes;
+  ~HostFilmBound() {
+    if (ctx->film_bytes > std::max(film, kKeepFilm)) {
+      cudaFree(ctx->d_film);
+      ctx->d_film = nullptr;
+      ctx->film_bytes = 0;
+    }
+    if (ctx->rgb_bytes > std::max(rgb, kKeepFilm)) {
+      cudaFree(ctx->d_rgb);
+      ctx->d_rgb = nullptr;
+      ctx->rgb_bytes = 0;
+    }
+  }
+};
 
 int32_t gyt_render(gyt_context* ctx, const gyt_scene* scene, const GytCamera* camera, const GytRenderParams* params,
                    float* rgb_out) {
@@ -4388,6 +4413,7 @@ int32_t gyt_render_light_tracing(gyt_context* ctx, const gyt_scene* scene, const
   if (!ctx || !scene || !camera || !rgb_out) return fail(ctx, GYT_ERR_INVALID, "light_tracing: null argument");
   const uint64_t npix = (uint64_t)camera->res_x * camera->res_y;
   GYT_CK(ctx, cudaSetDevice(ctx->device));
+  const HostFilmBound bound{ctx};
   int32_t st = ensure_host_films(ctx, 3 * std::max<uint64_t>(npix, 1) * sizeof(double), 3 * std::max<uint64_t>(npix, 1) * sizeof(float));
   if (st) return st;
   GYT_CK(ctx, cudaMemsetAsync(ctx->d_film, 0, 3 * npix * sizeof(double), ctx->stream));
@@ -4437,6 +4463,7 @@ int32_t gyt_render_volume(gyt_context* ctx, const gyt_scene* scene, const GytCam
   if (!ctx || !scene || !camera || !rgb_out) return fail(ctx, GYT_ERR_INVALID, "render_volume: null argument");
   const uint64_t npix = (uint64_t)camera->res_x * camera->res_y;
   GYT_CK(ctx, cudaSetDevice(ctx->device));
+  const HostFilmBound bound{ctx};
   int32_t st = ensure_host_films(ctx, 4 * std::max<uint64_t>(npix, 1) * sizeof(double), 3 * std::max<uint64_t>(npix, 1) * sizeof(float));
   if (st) return st;
   GYT_CK(ctx, cudaMemsetAsync(ctx->d_film, 0, 4 * npix * sizeof(double), ctx->stream));
@@ -4552,6 +4579,7 @@ int32_t gyt_film_quantize(gyt_context* ctx, const double* d_film, uint32_t res_x
   const uint64_t npix = (uint64_t)res_x * res_y;
   if (npix == 0 || npix > kPixMask) return fail(ctx, GYT_ERR_INVALID, "film_quantize: bad film size");
   GYT_CK(ctx, cudaSetDevice(ctx->device));
+  const HostFilmBound bound{ctx};
   int32_t st = ensure_host_films(ctx, 0, 3 * npix);
   if (st) return st;
   uint8_t* d = (uint8_t*)ctx->d_rgb;
@@ -4575,6 +4603,7 @@ int32_t gyt_film_save(gyt_context* ctx, const double* d_film, uint32_t res_x, ui
   bool ok = false;
   if (suffix == ".hdr") {
     GYT_CK(ctx, cudaSetDevice(ctx->device));
+    const HostFilmBound bound{ctx};
     const int32_t st = ensure_host_films(ctx, 0, 4 * npix);
     if (st) return st;
     uint8_t* d = (uint8_t*)ctx->d_rgb;

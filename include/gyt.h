@@ -133,7 +133,12 @@ typedef struct {
   uint64_t tri_tests[3];          /* triangle tests (counting mode only) */
 } GytProfile;
 
-/* Context on one CUDA device; owns a stream and the path-state pools. */
+/* Context on one CUDA device; owns a stream, the path-state pools and the
+ * device film and staging buffers of the calls that return host images or
+ * write files. Those buffers are kept between calls: by gyt_render and
+ * gyt_render_batch at their largest size, by the volumetric and light-tracing
+ * renders, gyt_film_quantize and gyt_film_save up to 128 MB each. All of it is
+ * given back by gyt_context_destroy. */
 int32_t gyt_context_create(int32_t device, gyt_context** out);
 void gyt_context_destroy(gyt_context* ctx);
 const char* gyt_last_error(const gyt_context* ctx);

@@ -1,5 +1,7 @@
 """Device memory that calls leave reserved on their context: as much as the
 next call of the kind needs, up to a bound. Needs a B200."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -10,6 +12,7 @@ from gyunity_b200 import scenes
 pytestmark = pytest.mark.gpu
 
 BLOCK = 2 << 20        # cudaMalloc takes device memory in blocks of 2 MB
+KEPT = 128 << 20       # what a context keeps of each film buffer (include/gyt.h)
 
 
 def _free():
@@ -50,3 +53,34 @@ def test_ray_queries_reserve_what_they_need(ctx2):
     sc.intersect(_rays(5))
     assert before - _free() == held
     sc.close()
+
+
+@pytest.mark.parametrize("call", ["light", "volume", "quantize"])
+def test_large_films_are_given_back(ctx2, call):
+    warm, c = ctx2
+
+    def run(ctx, res):
+        if call == "quantize":
+            film = torch.ones(res * res * 4, dtype=torch.float64, device="cuda")
+            ctx.film_quantize(film.data_ptr(), res, res)
+            del film
+            torch.cuda.empty_cache()
+            return
+        sd = scenes.cornell_box(res=16, spp=1) if call == "light" else scenes.cornell_fog(res=16, spp=1, max_depth=1)
+        cam = dataclasses.replace(sd.camera, res_x=res, res_y=res)
+        sc = g.Scene(sd, ctx)
+        film = g.Film(res, res)
+        camera = g.PinHoleCamera(film, cam.pos, cam.look_at, cam.up, cam.fovy, cam.film_distance)
+        integrator = g.LightTracing(1, 1) if call == "light" else g.VolPathTracing(1, 1)
+        g.Renderer(sc, camera, integrator).Render()
+        sc.close()
+
+    run(warm, 16)
+    run(c, 16)  # pools
+    before = _free()
+    run(c, 8000 if call == "quantize" else 3400)
+    # the colour sums and the staging buffer (quantize: the latter), each at most the bound
+    bound = KEPT if call == "quantize" else 2 * KEPT
+    assert before - _free() <= bound
+    run(c, 700)
+    assert before - _free() <= bound
