@@ -101,8 +101,12 @@ struct Queues {
   float4* madd; // per path slot: its MIS ray's contribution (k_connect; added by k_finish)
   float4* sx;  // adjoint pass, shadow ray: material bits, d log f / d alpha, light bits, -
   float4* mx;  // adjoint pass, MIS ray: material bits, d log f / d alpha, -, -
-  float4* pc;  // adjoint pass, path slot: the last continuation's contribution, material | kPendValid bits
-  float* pa;   // adjoint pass, path slot: its d log f / d alpha
+  // adjoint pass, path slot: the last continuation's contribution with material
+  // | kPendValid bits, and its d log f / d alpha. k_shade_adj leaves them for
+  // k_grad_adj in the replay state of the next iteration (AdjBuf::delta and
+  // pend), which holds nothing until k_finish_adj.
+  float4* pc;
+  float* pa;
 };
 
 // Adjoint (path replay) state per path slot, ping-ponged with the pool.
@@ -3522,8 +3526,6 @@ int32_t ensure_adj(gyt_context* ctx) {
   }
   GYT_CK(ctx, dalloc(L, &ctx->q.sx, n));
   GYT_CK(ctx, dalloc(L, &ctx->q.mx, n));
-  GYT_CK(ctx, dalloc(L, &ctx->q.pc, n));
-  GYT_CK(ctx, dalloc(L, &ctx->q.pa, n));
   ctx->adj_cap = ctx->pool_cap;
   return GYT_OK;
 }
@@ -3659,9 +3661,12 @@ int32_t run_adjoint(gyt_context* ctx, const gyt_scene* scene, const Cam& cam, co
     return launch_next(s, grid_for(n_new), k_generate_adj, ctx->pool[cur], ctx->adj[cur], base, n_new, first, cam, p->spp,
                        d_list, tab, in);
   };
-  auto iterate = [&](int cur, Live live, uint32_t bound, const Queues& q, uint32_t* launches) {
+  auto iterate = [&](int cur, Live live, uint32_t bound, const Queues& q0, uint32_t* launches) {
     const PathBuf P = ctx->pool[cur], N = ctx->pool[cur ^ 1];
     const AdjBuf A = ctx->adj[cur], AN = ctx->adj[cur ^ 1];
+    Queues q = q0;
+    q.pc = AN.delta;
+    q.pa = (float*)AN.pend;
     launch_next(s, trace_grid(g_ext, bound), W == 8 ? k_extend<8, false> : k_extend<2, false>, P, live, D, q.hit,
                 q.counts + 2, nullptr);
     launch_next(s, grid_for(bound), shade, P, A, live, D, prm, q, tab, G);

@@ -1,5 +1,6 @@
 """Device memory that calls leave reserved on their context: as much as the
-next call of the kind needs, up to a bound. Needs a B200."""
+next call of the kind needs, up to a bound, and no more per path slot of the
+adjoint pass than its state takes. Needs a B200."""
 import dataclasses
 
 import numpy as np
@@ -53,6 +54,28 @@ def test_ray_queries_reserve_what_they_need(ctx2):
     sc.intersect(_rays(5))
     assert before - _free() == held
     sc.close()
+
+
+def test_adjoint_state_per_path_slot():
+    torch.cuda.init()
+    cap = 1 << 22
+    c = g.Context(0, capacity=cap)
+    p = scenes.inverse_params(groups=4, seed=1)
+    sd = scenes.inverse_box(p, level=3, res=32, spp=2, max_depth=4, rr_depth=4)
+    sc = g.Scene(sd, c)
+    k = np.arange(200)
+    xys = np.stack([k % 32, k // 32, k % 2], 1).astype(np.uint32)
+    L = sc.trace_paths(xys)[0]
+    warm = g.Context(0, capacity=1024)  # loads the adjoint pass's kernels
+    warm.diff_backward_paths(g.Scene(sd, warm), xys, np.ones((200, 3)), L)
+    before = _free()
+    c.diff_backward_paths(sc, xys, np.ones((200, 3)), L)
+    # per slot two copies of the replay state (adjoint weight, primal radiance,
+    # pending continuation: 16 + 16 + 8) and the payload of two rays (16 each)
+    assert before - _free() <= cap * (2 * 40 + 32) + 8 * BLOCK
+    warm.close()
+    sc.close()
+    c.close()
 
 
 @pytest.mark.parametrize("call", ["light", "volume", "quantize"])
