@@ -1443,9 +1443,12 @@ GYT_D void film_add(double* film, uint32_t w, uint32_t x, uint32_t y, float3 L) 
 
 // Finished paths go to the film (FP64 atomics, Film::AddSample with the box
 // filter, visual/Film.h:61-87); live paths are compacted into the next pool.
+// madd is written by the kernel before this one, which may still run when this
+// one starts: not const __restrict__, which promises that it is read-only for
+// as long as the kernel lives.
 __global__ void __launch_bounds__(kBlock) k_finish(PathBuf cur, PathBuf nxt, Live live, double* __restrict__ film,
                                                    uint32_t res_x, uint32_t* __restrict__ counter,
-                                                   const float4* __restrict__ madd, DebugOut dbg) {
+                                                   const float4* madd, DebugOut dbg) {
   chain_start();
   const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1699,8 +1702,7 @@ __global__ void __launch_bounds__(kBlock) k_grad_adj(AdjBuf A, Live live, DevSce
 // Live paths (and their adjoint state) compacted; finished paths are done
 // (their gradient was moved at their last bounce).
 __global__ void __launch_bounds__(kBlock) k_finish_adj(PathBuf cur, PathBuf nxt, AdjBuf A, AdjBuf AN, Live live,
-                                                       uint32_t* __restrict__ counter,
-                                                       const float4* __restrict__ madd) {
+                                                       uint32_t* __restrict__ counter, const float4* madd) {
   chain_start();
   const uint32_t n = live.get();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
