@@ -2949,15 +2949,19 @@ struct gyt_context {
   unsigned long long* d_counters = nullptr;  // node visits and triangle tests per traversal kernel
   GytProfile prof = {};
   int sms = 0;
-  // batched renders: device loop state, configuration and the captured graph
-  // (rebuilt when its kernels' arguments change)
+  // batched renders: device loop state, configuration and the captured graphs,
+  // one of batches without and one of batches with an environment light (their
+  // shade kernels differ): a program that alternates keeps both. Each is rebuilt
+  // when its kernels or their arguments change.
   IterState* d_iter = nullptr;
   IterState* h_iter = nullptr;  // pinned
   GytBatchConfig bcfg = {0, 0, 0, 1, 0};
   int btrace[2][2] = {};  // occupancy limit (blocks per SM) of the batched extend/shadow, width 2/8
-  cudaGraph_t bgraph = nullptr;
-  cudaGraphExec_t bexec = nullptr;
-  uint64_t bkey[6] = {};
+  struct BatchGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    uint64_t key[6] = {};
+  } bgraphs[2];
   // adjoint pass: replay state per path slot (two buffers) and queue payloads
   AdjBuf adj[2] = {};
   uint32_t adj_cap = 0;
@@ -3784,8 +3788,10 @@ void gyt_context_destroy(gyt_context* c) {
   cudaFree(c->d_film);
   cudaFree(c->d_rgb);
   cudaFree(c->d_query);
-  if (c->bexec) cudaGraphExecDestroy(c->bexec);
-  if (c->bgraph) cudaGraphDestroy(c->bgraph);
+  for (auto& bg : c->bgraphs) {
+    if (bg.exec) cudaGraphExecDestroy(bg.exec);
+    if (bg.graph) cudaGraphDestroy(bg.graph);
+  }
   if (c->d_iter) cudaFree(c->d_iter);
   if (c->h_iter) cudaFreeHost(c->h_iter);
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -4958,7 +4964,7 @@ namespace {
 struct BatchPlan {
   int W = 2;
   int sampler = -1;  // 0 / 1: every instance samples with Sobol' / Halton (the shade kernel compiled for it)
-  bool env = true;   // some instance has an environment light
+  bool env = true;   // the shade kernel with the environment light
   uint32_t stride_grid = 0, ext_grid = 0, sh_grid = 0, shade_grid = 0;
 };
 
@@ -5015,17 +5021,18 @@ constexpr uint32_t kKernelsPerHalf = 7;
 // The batched render as one graph: a while-loop node whose body is two
 // half-iterations (pool 0 -> 1 -> 0); k_batch_end sets the loop condition.
 int32_t ensure_batch_graph(gyt_context* ctx, const BatchPlan& b) {
-  const uint64_t key[6] = {(uint64_t)b.W | ((uint64_t)(b.sampler + 1) << 8) | ((uint64_t)b.env << 16), (uint64_t)b.stride_grid,
+  auto& bg = ctx->bgraphs[b.env ? 1 : 0];
+  const uint64_t key[6] = {(uint64_t)b.W | ((uint64_t)(b.sampler + 1) << 8), (uint64_t)b.stride_grid,
                            ((uint64_t)b.ext_grid << 32) | b.sh_grid, (uint64_t)b.shade_grid,
                            (uint64_t)(uintptr_t)ctx->pool[0].o, (uint64_t)ctx->pool_cap};
-  if (ctx->bexec && std::memcmp(key, ctx->bkey, sizeof(key)) == 0) return GYT_OK;
-  if (ctx->bexec) cudaGraphExecDestroy(ctx->bexec);
-  if (ctx->bgraph) cudaGraphDestroy(ctx->bgraph);
-  ctx->bexec = nullptr;
-  ctx->bgraph = nullptr;
+  if (bg.exec && std::memcmp(key, bg.key, sizeof(key)) == 0) return GYT_OK;
+  if (bg.exec) cudaGraphExecDestroy(bg.exec);
+  if (bg.graph) cudaGraphDestroy(bg.graph);
+  bg.exec = nullptr;
+  bg.graph = nullptr;
   cudaGraph_t g = nullptr;
   GYT_CK(ctx, cudaGraphCreate(&g, 0));
-  ctx->bgraph = g;
+  bg.graph = g;
   cudaGraphConditionalHandle cond;
   GYT_CK(ctx, cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault));
   cudaGraphNodeParams np = {};
@@ -5048,8 +5055,8 @@ int32_t ensure_batch_graph(gyt_context* ctx, const BatchPlan& b) {
   }
   cudaGraphExec_t ex = nullptr;
   GYT_CK(ctx, cudaGraphInstantiate(&ex, g, 0));
-  ctx->bexec = ex;
-  std::memcpy(ctx->bkey, key, sizeof(key));
+  bg.exec = ex;
+  std::memcpy(bg.key, key, sizeof(key));
   return GYT_OK;
 }
 
@@ -5113,7 +5120,7 @@ int32_t run_batch(gyt_context* ctx, const BatchInput& in, GytRenderStats* stats)
   int sampler = in.insts.empty() ? 0 : (int)in.insts[0].prm.sampler;
   for (const Inst& I : in.insts)
     if ((int)I.prm.sampler != sampler) sampler = -1;
-  bool env = false;
+  bool env = sampler < 0;  // the kernel of mixed samplers has the environment light
   for (const Inst& I : in.insts) env = env || I.s.has_env;
   const BatchPlan b = batch_plan(ctx, in.W, sampler, env);
   std::lock_guard<std::mutex> lock(g_batch_mutex);
@@ -5146,7 +5153,7 @@ int32_t run_batch(gyt_context* ctx, const BatchInput& in, GytRenderStats* stats)
     *ctx->h_iter = is;
     GYT_CK(ctx, cudaMemcpyAsync(ctx->d_iter, ctx->h_iter, sizeof(IterState), cudaMemcpyHostToDevice, s));
     if (graph) {
-      GYT_CK(ctx, cudaGraphLaunch(ctx->bexec, s));
+      GYT_CK(ctx, cudaGraphLaunch(ctx->bgraphs[b.env ? 1 : 0].exec, s));
     } else if (prof) {
       // one half at a time, every kernel between events; profile slots as
       // gyt_render_device fills them (3 = connect, 4 unused)
