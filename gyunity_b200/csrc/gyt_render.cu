@@ -705,10 +705,7 @@ GYT_D void pooled_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load
       if (ri >= 0) {
         if (BATCH) tv.node(lg, rc, o, tmax);
         else tv.node(s, rc, o, tmax);
-        if (COUNT) {
-          cnt.nodes++;
-          cnt.tris += __popc(tv.tmask);
-        }
+        if (COUNT) cnt.nodes++;
       } else {
         tv.tmask = 0u;
       }
@@ -767,6 +764,8 @@ GYT_D void pooled_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load
         // this lane's tests of the round
         const uint32_t took = own ? min(c, 32u - off) : 0u;
         const uint32_t seg = took ? (kAll >> (32u - took)) << off : 0u;
+        // counted as in order: an any-hit ray's up to its first hit
+        if (COUNT) cnt.tris += ANY && (hits & seg) ? (uint32_t)__ffs(hits & seg) - off : took;
         if (ANY) {
           if (hits & seg) occluded = true;
         } else if (hits) {
