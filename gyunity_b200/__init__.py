@@ -209,6 +209,14 @@ class Context:
         self.check(self._lib.gyt_bsdf_table(self.handle, n, _c.ptr(t), _c.ptr(p), _c.ptr(v), _c.ptr(out)))
         return out
 
+    def normalize(self, xyz, length):
+        """gyt_normalize: the GPU's Vector::Norm of (n, 3) vectors, and their
+        quotients by the given lengths as it divides."""
+        x = np.ascontiguousarray(np.concatenate([np.reshape(xyz, (-1, 3)), np.reshape(length, (-1, 1))], 1), np.float32)
+        out = np.empty((x.shape[0], 6), np.float32)
+        self.check(self._lib.gyt_normalize(self.handle, x.shape[0], _c.ptr(x), _c.ptr(out)))
+        return out[:, :3], out[:, 3:]
+
     def sobol(self, dims, indices):
         """sobol::sample (sampler/Sobol.h:46-61) for (dimension, index) pairs."""
         d = np.ascontiguousarray(dims, np.uint32)

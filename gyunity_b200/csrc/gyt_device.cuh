@@ -30,27 +30,31 @@ GYT_HD float length(float3 a) { return sqrtf(dot(a, a)); }
 GYT_HD float3 norm_in(float3 a) { return a / length(a); }
 // The same, out of line on the device: a bounce normalises about twenty
 // vectors, the shade kernels are bound by instruction fetch (every warp walks
-// 130 KB of code about once), and a called copy stays in the instruction cache.
+// 105 KB of code about once), and a called copy stays in the instruction cache.
+// Mesh at 16 spp, shade launches of a render: 16.5 ms inlined with
+// nine-operation divisions, 14.9 ms called.
+//
 // Its three quotients share y = RN(1 / s): q = RN(a y), then one correction
 // q - RN(q s - a) y rounds as a / s does. Markstein (1990): with y correctly
 // rounded that holds unless a / s lies within 1.5 * 2^-24 ulp of a rounding
-// boundary; all such pairs of 24-bit significands (17.4M, from m s + d = 0 mod
-// 2^24 for |d| <= 3) were checked to round correctly as well. Lengths outside
-// [2^-60, 2^60] divide plainly; a component below 2^-100, whose residual may be
-// subnormal, can be off by one ulp of its own. The sign of the residual keeps
-// that of a zero component. Mesh at 16 spp, shade launches of a render: 16.5
-// ms inlined with nine-operation divisions, 14.9 ms called.
-#ifdef __CUDA_ARCH__
+// boundary, and all such pairs of 24-bit significands (22.3M) round correctly as
+// well (tests/test_gpu_normalize.py runs them). It needs q normal and q s - a
+// exact: components and lengths of [2^-60, 2^60], and zeros, whose sign the
+// sign of the residual keeps; all else (a length bounds its components, so one
+// comparison each way) divides plainly.
 __device__ __noinline__ float3 norm_plain(float x, float y, float z, float s) { return mk(x / s, y / s, z / s); }
-__device__ __noinline__ float3 norm_call(float x, float y, float z) {
-  const float s = length(mk(x, y, z));  // bounds every component
-  if (!(s < 1.152921504606847e18f && s > 8.673617379884035e-19f)) return norm_plain(x, y, z, s);
+GYT_D float3 norm_div(float x, float y, float z, float s) {
+  // twice the bits drop the sign; zeros wrap to the top
+  const uint32_t low = min(min(2u * __float_as_uint(x) - 2u, 2u * __float_as_uint(y) - 2u), 2u * __float_as_uint(z) - 2u);
+  if (!(s <= 0x1p60f && low >= 2u * 0x21800000u - 2u)) return norm_plain(x, y, z, s);
   const float r = __frcp_rn(s);
   const float qx = __fmul_rn(x, r), qy = __fmul_rn(y, r), qz = __fmul_rn(z, r);
   return mk(__fmaf_rn(-__fmaf_rn(qx, s, -x), r, qx), __fmaf_rn(-__fmaf_rn(qy, s, -y), r, qy),
             __fmaf_rn(-__fmaf_rn(qz, s, -z), r, qz));
 }
-#endif
+__device__ __noinline__ float3 norm_call(float x, float y, float z) {
+  return norm_div(x, y, z, length(mk(x, y, z)));  // the length bounds every component
+}
 GYT_HD float3 norm(float3 a) {
 #ifdef __CUDA_ARCH__
   return norm_call(a.x, a.y, a.z);

@@ -2820,6 +2820,17 @@ __global__ void k_bsdf_table(uint64_t n, const float* __restrict__ params, const
   o[7] = fe.x; o[8] = fe.y; o[9] = fe.z; o[10] = pe;
 }
 
+// Vector::Norm as the shading kernels call it, and its quotients by a given
+// length: 4 floats in (x y z s), 6 out.
+__global__ void k_normalize(uint64_t n, const float4* v, float* out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 a = v[i];
+  const float3 u = norm(f3(a)), q = norm_div(a.x, a.y, a.z, a.w);
+  float* o = out + 6 * i;
+  o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = q.x; o[4] = q.y; o[5] = q.z;
+}
+
 __global__ void k_sobol(SamplerTables tab, uint64_t n, const uint32_t* dims, const uint64_t* idx, float* out) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -4850,6 +4861,27 @@ int32_t gyt_bsdf_table(gyt_context* ctx, uint64_t n, const uint32_t* types, cons
   GYT_CK(ctx, cudaGetLastError());
   GYT_CK(ctx, cudaStreamSynchronize(ctx->stream));
   GYT_CK(ctx, cudaMemcpy(out, dout, 11 * n * 4, cudaMemcpyDeviceToHost));
+  return GYT_OK;
+}
+
+int32_t gyt_normalize(gyt_context* ctx, uint64_t n, const float* xyzs, float* out) {
+  if (!ctx || (n && (!xyzs || !out))) return fail(ctx, GYT_ERR_INVALID, "normalize: null argument");
+  if (n == 0) return GYT_OK;
+  GYT_CK(ctx, cudaSetDevice(ctx->device));
+  std::vector<void*> tmp;
+  struct Guard {
+    std::vector<void*>& v;
+    ~Guard() { for (void* p : v) cudaFree(p); }
+  } guard{tmp};
+  float4* dv = nullptr;
+  float* dout = nullptr;
+  GYT_CK(ctx, dalloc(tmp, &dv, n));
+  GYT_CK(ctx, dalloc(tmp, &dout, 6 * n));
+  GYT_CK(ctx, cudaMemcpyAsync(dv, xyzs, n * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
+  k_normalize<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, dv, dout);
+  GYT_CK(ctx, cudaGetLastError());
+  GYT_CK(ctx, cudaStreamSynchronize(ctx->stream));
+  GYT_CK(ctx, cudaMemcpy(out, dout, 6 * n * sizeof(float), cudaMemcpyDeviceToHost));
   return GYT_OK;
 }
 

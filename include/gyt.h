@@ -234,6 +234,12 @@ int32_t gyt_sobol(gyt_context* ctx, uint64_t n, const uint32_t* dims, const uint
 int32_t gyt_bsdf_table(gyt_context* ctx, uint64_t n, const uint32_t* types, const float* params, const float* vec,
                        float* out);
 
+/* Vector::Norm (math/Linagl.h:527-531) on the GPU for n vectors, and its three
+ * quotients by a given length: xyzs[4 i..] = x, y, z and a length s of at least
+ * |x|, |y| and |z|; out[6 i..] = Norm(x, y, z), then x / s, y / s, z / s as the
+ * kernels' normalisation divides (correctly rounded). For parity tests. */
+int32_t gyt_normalize(gyt_context* ctx, uint64_t n, const float* xyzs, float* out);
+
 /* SobolEnum::GetIndex (sampler/SobolEnum.h:23-28) for n (s, x, y) triplets. */
 int32_t gyt_sobol_enum_index(gyt_context* ctx, uint32_t res_x, uint32_t res_y, uint64_t n,
                              const uint32_t* sxy, uint64_t* out);
