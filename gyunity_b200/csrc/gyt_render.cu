@@ -530,10 +530,6 @@ GYT_D int trace(const DevScene& s, float3 o, float3 d, float& tmax, float& b1, f
   return prim;
 }
 
-template <bool ANY, bool COUNT, bool BATCH, bool CLS, class Load, class Done>
-GYT_D void pooled_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load, Done done,
-                        unsigned long long* counters);
-
 // Persistent traversal with dynamic ray fetching: every lane of a warp keeps
 // a ray; lanes whose ray is finished take new ray indices before the next
 // traversal step (one atomicAdd per warp), so warps stay full until the
@@ -542,27 +538,23 @@ GYT_D void pooled_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load
 // load(i, o, d, tmax) fetches ray i; done(i, prim, tmax, b1, b2) consumes
 // its result.
 //
-// Two traversal steps between fetch checks keep the ballot cost small (a
-// binary step already walks down to a leaf). The 8-wide BVH's kernels are
-// pooled_trace.
+// Over the binary BVH every lane tests its own triangles. Two traversal steps
+// between fetch checks keep the ballot cost small (a step already walks down to
+// a leaf).
 //
 // BATCH: every ray carries its own geometry (load fills the lane's TraceGeo);
 // otherwise all rays use the scene s. CLS: triangle hits carry their shading
 // class (test_tris).
-template <int W, bool ANY, bool COUNT, bool BATCH = false, bool CLS = false, class Load, class Done>
-GYT_D void persistent_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load, Done done,
-                            unsigned long long* counters) {
-  if constexpr (W == 8) {
-    pooled_trace<ANY, COUNT, BATCH, CLS>(s, next, n, load, done, counters);
-    return;
-  }
+template <bool ANY, bool COUNT, bool BATCH, bool CLS, class Load, class Done>
+GYT_D void binary_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load, Done done,
+                        unsigned long long* counters) {
   const uint32_t lane = threadIdx.x & 31u;
   int ri = -1;  // -1 idle, -2 queue exhausted
   float3 o = mk(0.f, 0.f, 0.f), d = o;
   float tmax = 0.f, b1 = 0.f, b2 = 0.f;
   int prim = -1;
   RayConst rc;
-  typename TraversalOf<W>::type tv;
+  BinaryTraversal tv;
   TraceCount cnt;
   TraceGeo lg{};  // the lane's geometry (BATCH)
   for (;;) {
@@ -636,7 +628,7 @@ GYT_D void persistent_trace(const DevScene& s, uint32_t* next, uint32_t n, Load 
 __shared__ float4 g_ray[kSlabWarps][2][32];
 __shared__ uint32_t g_best[kSlabWarps][32], g_owner[kSlabWarps][32];
 
-// persistent_trace over the 8-wide BVH with the warp's triangle tests pooled:
+// The same over the 8-wide BVH with the warp's triangle tests pooled:
 // after every node step the lanes' hit triangles, about one each but four to
 // six on some lane, are dealt out one per lane, whichever ray they belong to.
 // Tested by their own lanes they ran at a few lanes of 32 (11 threads per
@@ -817,6 +809,13 @@ GYT_D void pooled_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load
       atomicAdd(counters + 1, tris);
     }
   }
+}
+
+template <int W, bool ANY, bool COUNT, bool BATCH = false, bool CLS = false, class Load, class Done>
+GYT_D void persistent_trace(const DevScene& s, uint32_t* next, uint32_t n, Load load, Done done,
+                            unsigned long long* counters) {
+  if constexpr (W == 8) pooled_trace<ANY, COUNT, BATCH, CLS>(s, next, n, load, done, counters);
+  else binary_trace<ANY, COUNT, BATCH, CLS>(s, next, n, load, done, counters);
 }
 
 // Hit triangle k in leaf order: positions, shading normals, face normal
