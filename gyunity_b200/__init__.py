@@ -209,6 +209,18 @@ class Context:
         self.check(self._lib.gyt_bsdf_table(self.handle, n, _c.ptr(t), _c.ptr(p), _c.ptr(v), _c.ptr(out)))
         return out
 
+    def bsdf_directions(self, types, params, wo, u):
+        """gyt_bsdf_directions: for n cases (kind, 16 parameters, wo, u) the
+        sampled wi and its pdf, and the direction sampled on its own with
+        whether the sample is valid."""
+        t = np.ascontiguousarray(types, np.uint32)
+        n = t.shape[0]
+        p = np.ascontiguousarray(params, np.float32).reshape(n, 16)
+        v = np.ascontiguousarray(np.concatenate([np.reshape(wo, (n, 3)), np.reshape(u, (n, 3))], 1), np.float32)
+        out = np.empty((n, 8), np.float32)
+        self.check(self._lib.gyt_bsdf_directions(self.handle, n, _c.ptr(t), _c.ptr(p), _c.ptr(v), _c.ptr(out)))
+        return out[:, :3], out[:, 3], out[:, 4:7], out[:, 7] != 0
+
     def normalize(self, xyz, length):
         """gyt_normalize: the GPU's Vector::Norm of (n, 3) vectors, and their
         quotients by the given lengths as it divides."""

@@ -27,7 +27,7 @@ EXPORTS = ["gyt_context_create", "gyt_context_destroy", "gyt_last_error", "gyt_c
            "gyt_mesh_load_obj", "gyt_mesh_size", "gyt_mesh_read", "gyt_mesh_transform", "gyt_mesh_destroy",
            "gyt_render_device_noalloc", "gyt_context_set_batch_config", "gyt_context_get_batch_config",
            "gyt_render_batch_device", "gyt_render_batch", "gyt_batch_autotune", "gyt_scene_set_materials",
-           "gyt_scene_freeze_sampling", "gyt_scene_read_wide_bvh", "gyt_bsdf_table", "gyt_normalize",
+           "gyt_scene_freeze_sampling", "gyt_scene_read_wide_bvh", "gyt_bsdf_table", "gyt_normalize", "gyt_bsdf_directions",
            "gyt_diff_forward", "gyt_diff_backward", "gyt_diff_backward_paths"]
 
 # BVH builders (GYT_BVH_BUILD_* in include/gyt.h)
@@ -158,6 +158,7 @@ def load():
     L.gyt_scene_set_materials.argtypes = [P, P, P, U32]
     L.gyt_scene_freeze_sampling.argtypes = [P, P]
     L.gyt_bsdf_table.argtypes = [P, U64, P, P, P, P]
+    L.gyt_bsdf_directions.argtypes = [P, U64, P, P, P, P]
     L.gyt_normalize.argtypes = [P, U64, P, P]
     L.gyt_diff_forward.argtypes = [P, P, ctypes.POINTER(GytCamera), ctypes.POINTER(GytRenderParams), P, P,
                                    ctypes.POINTER(GytRenderStats)]

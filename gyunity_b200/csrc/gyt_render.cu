@@ -2819,6 +2819,25 @@ __global__ void k_bsdf_table(uint64_t n, const float* __restrict__ params, const
   o[7] = fe.x; o[8] = fe.y; o[9] = fe.z; o[10] = pe;
 }
 
+// A sample of each case's BxDF and its direction alone, by the two functions the
+// shading kernels call, in the frame of the coordinate axes: 6 floats in (wo, u),
+// 8 out (wi, pdf; direction, 1 unless void).
+__global__ void k_bsdf_directions(uint64_t n, const float* __restrict__ params, const uint32_t* __restrict__ types,
+                                  const float* __restrict__ vec, float* __restrict__ out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float* v = vec + 6 * i;
+  const float3 wo = mk(v[0], v[1], v[2]), z = mk(0.f, 0.f, 1.f);
+  const Bsdf b{load_lobe(params, types, (uint32_t)i), mk(1.f, 0.f, 0.f), mk(0.f, 1.f, 0.f), z, z};
+  float3 wi = mk(0.f, 0.f, 0.f), wd = wi;
+  float pdf = 0.f;
+  b.sample(wo, &wi, &pdf, v[3], v[4], v[5]);
+  const bool ok = b.sample_dir(wo, &wd, v[3], v[4], v[5]);
+  float* o = out + 8 * i;
+  o[0] = wi.x; o[1] = wi.y; o[2] = wi.z; o[3] = pdf;
+  o[4] = wd.x; o[5] = wd.y; o[6] = wd.z; o[7] = ok ? 1.f : 0.f;
+}
+
 // Vector::Norm as the shading kernels call it, and its quotients by a given
 // length: 4 floats in (x y z s), 6 out.
 __global__ void k_normalize(uint64_t n, const float4* v, float* out) {
@@ -4860,6 +4879,35 @@ int32_t gyt_bsdf_table(gyt_context* ctx, uint64_t n, const uint32_t* types, cons
   GYT_CK(ctx, cudaGetLastError());
   GYT_CK(ctx, cudaStreamSynchronize(ctx->stream));
   GYT_CK(ctx, cudaMemcpy(out, dout, 11 * n * 4, cudaMemcpyDeviceToHost));
+  return GYT_OK;
+}
+
+int32_t gyt_bsdf_directions(gyt_context* ctx, uint64_t n, const uint32_t* types, const float* params, const float* vec,
+                            float* out) {
+  if (!ctx || (n && (!types || !params || !vec || !out))) return fail(ctx, GYT_ERR_INVALID, "bsdf_directions: null argument");
+  if (n == 0) return GYT_OK;
+  if (n >= (1ull << 32)) return fail(ctx, GYT_ERR_UNSUPPORTED, "bsdf_directions: more than 2^32 cases");
+  for (uint64_t i = 0; i < n; ++i)
+    if (types[i] > GYT_MAT_DIELECTRIC) return fail(ctx, GYT_ERR_INVALID, "bsdf_directions: unknown material kind");
+  GYT_CK(ctx, cudaSetDevice(ctx->device));
+  std::vector<void*> tmp;
+  struct Guard {
+    std::vector<void*>& v;
+    ~Guard() { for (void* p : v) cudaFree(p); }
+  } guard{tmp};
+  uint32_t* dt = nullptr;
+  float *dp = nullptr, *dv = nullptr, *dout = nullptr;
+  GYT_CK(ctx, dalloc(tmp, &dt, n));
+  GYT_CK(ctx, dalloc(tmp, &dp, 16 * n));
+  GYT_CK(ctx, dalloc(tmp, &dv, 6 * n));
+  GYT_CK(ctx, dalloc(tmp, &dout, 8 * n));
+  GYT_CK(ctx, cudaMemcpyAsync(dt, types, n * 4, cudaMemcpyHostToDevice, ctx->stream));
+  GYT_CK(ctx, cudaMemcpyAsync(dp, params, 16 * n * 4, cudaMemcpyHostToDevice, ctx->stream));
+  GYT_CK(ctx, cudaMemcpyAsync(dv, vec, 6 * n * 4, cudaMemcpyHostToDevice, ctx->stream));
+  k_bsdf_directions<<<grid_for(n), kBlock, 0, ctx->stream>>>(n, dp, dt, dv, dout);
+  GYT_CK(ctx, cudaGetLastError());
+  GYT_CK(ctx, cudaStreamSynchronize(ctx->stream));
+  GYT_CK(ctx, cudaMemcpy(out, dout, 8 * n * 4, cudaMemcpyDeviceToHost));
   return GYT_OK;
 }
 

@@ -234,6 +234,13 @@ int32_t gyt_sobol(gyt_context* ctx, uint64_t n, const uint32_t* dims, const uint
 int32_t gyt_bsdf_table(gyt_context* ctx, uint64_t n, const uint32_t* types, const float* params, const float* vec,
                        float* out);
 
+/* The direction alone of BxDF::Sample as the MIS half of direct lighting takes
+ * it first: vec[6 i..] = wo, u; out[8 i..] = wi and pdf of the whole sample (wi
+ * is arbitrary where pdf is 0), then the direction on its own and 1, or 0 where
+ * the sample is void. For parity tests. */
+int32_t gyt_bsdf_directions(gyt_context* ctx, uint64_t n, const uint32_t* types, const float* params, const float* vec,
+                            float* out);
+
 /* Vector::Norm (math/Linagl.h:527-531) on the GPU for n vectors, and its three
  * quotients by a given length: xyzs[4 i..] = x, y, z and a length s of at least
  * |x|, |y| and |z|; out[6 i..] = Norm(x, y, z), then x / s, y / s, z / s as the
