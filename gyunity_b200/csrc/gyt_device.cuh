@@ -29,10 +29,10 @@ GYT_HD float length(float3 a) { return sqrtf(dot(a, a)); }
 // Vector::Norm divides by the length (math/Linagl.h:527-531)
 GYT_HD float3 norm_in(float3 a) { return a / length(a); }
 // The same, out of line on the device: a bounce normalises about twenty
-// vectors, the shade kernels are bound by instruction fetch (every warp walks
-// 105 KB of code about once), and a called copy stays in the instruction cache.
-// Mesh at 16 spp, shade launches of a render: 16.5 ms inlined with
-// nine-operation divisions, 14.9 ms called.
+// vectors, every warp of a shade kernel walks its code (130 KB then, 105 KB now
+// without an environment light) about once, and a called copy stays in the
+// instruction cache. Mesh at 16 spp, shade launches of a render: 16.5 ms inlined
+// with nine-operation divisions, 14.9 ms called.
 //
 // Its three quotients share y = RN(1 / s): q = RN(a y), then one correction
 // q - RN(q s - a) y rounds as a / s does. Markstein (1990): with y correctly
@@ -901,8 +901,8 @@ struct Bsdf {
     return mk(0.f, 0.f, 0.f);
   }
   // Not inlined: the shading kernels sample the BSDF at two or three places,
-  // and one out-of-line copy keeps their instruction footprint small (they are
-  // bound by instruction fetch).
+  // and one out-of-line copy keeps their instruction footprint small (each warp
+  // fetches most of the kernel's code once).
   __device__ __noinline__ bool sample_dir(float3 wo, float3* wi, float u0, float u1, float u2) const {
     const Lobe::Dir r = lobe.sample_dir(local(wo), u0, u1, u2);
     *wi = world(r.wi);

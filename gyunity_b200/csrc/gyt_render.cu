@@ -202,12 +202,14 @@ template <int W>
 constexpr int shadow_blocks_per_sm() { return 4; }
 template <int W>
 constexpr int extend_blocks_per_sm() { return 5; }
-// The shade kernels, once their blocks are sorted by lobe type, are bound by
-// instruction fetch and latency: 64 registers (four blocks of 256, some
-// spilled values) shade the mesh in 13.5 ms a render, 80 registers (three
-// blocks) in 0.9 ms more, 48 (five) in 1.5 more. The block is also what keeps
-// eight warps on the same code: warps that sort a window of their own and run
-// on independently, with every warp slot of the SM filled, took 20% longer.
+// The shade kernels, once their blocks are sorted by lobe type, are bound by the
+// latency of their loads, spilled values among them, then by instruction fetch
+// (7.0 and 1.5 warps stalled per issue on a full pool of the uneven batch): 64
+// registers (four blocks of 256, some spilled values) shade the mesh in 13.5 ms
+// a render, 80 registers (three blocks) in 0.9 ms more, 48 (five) in 1.5 more.
+// The block is also what keeps eight warps on the same code: warps that sort a
+// window of their own and run on independently, with every warp slot of the SM
+// filled, took 20% longer.
 constexpr int kShadeBlocksPerSm = 4;
 
 // meta bit 20: the bounce queued an MIS ray whose contribution k_finish adds
@@ -631,9 +633,10 @@ __shared__ uint32_t g_best[kSlabWarps][32], g_owner[kSlabWarps][32];
 // The same over the 8-wide BVH with the warp's triangle tests pooled:
 // after every node step the lanes' hit triangles, about one each but four to
 // six on some lane, are dealt out one per lane, whichever ray they belong to.
-// Tested by their own lanes they ran at a few lanes of 32 (11 threads per
-// instruction over the whole kernel; 19 now, 1.3 to 2 rounds of about 20 tests
-// a step). A lane's triangles keep their order and equal distances go to the
+// Tested by their own lanes they ran at a few lanes of 32 (a full pool of the
+// uneven batch: 12.7 threads per instruction over the closest-hit kernel, 11.5
+// over the shadow kernel; 20.4 and 16.0 now, 1.3 to 2 rounds of about 20 tests a
+// step). A lane's triangles keep their order and equal distances go to the
 // later one, as in the sequential test, so hits are the same. With the node
 // test below, closest hits and shadow rays of a render: mesh (1024x1024, 16
 // spp) 15.3 -> 12.7 and 11.8 -> 10.2 ms, glass knot under a sky 4.6 -> 3.8 and
@@ -2426,9 +2429,11 @@ GYT_D void vpt_direct_queue(const DevScene& s, const Queues& q, const VPoint& p,
 // shadow segment. The light point is recomputed from its two numbers where it
 // is used rather than kept.
 //
-// Two blocks per SM (128 registers, no spills): the kernel is bound by
-// instruction fetch, and three or four blocks with spilled values are 2 to 4%
-// slower (the fogged box 6.04 against 5.93 ms a render).
+// Two blocks per SM (128 registers; three of the four builds spill nothing, one 4
+// bytes): the kernel is bound by divergence (13 of 32 lanes run) and dependent
+// instructions at 45% of the issue slots, and three or four blocks, whose
+// spilled values add instructions, are 2 to 4% slower (the fogged box 6.04
+// against 5.93 ms a render).
 template <int SAMPLER, bool EQUI>
 __global__ void __launch_bounds__(kBlock, 2) k_vshade(PathBuf cur, Live live, DevScene s, Params prm,
                                                                  Queues q, SamplerTables tab) {
@@ -3379,9 +3384,11 @@ inline uint32_t trace_grid(int full, uint32_t n) { return std::min((uint32_t)ful
 // which they are: an iteration's grid is sized for the first one's count, so
 // the blocks past the live paths, which end at once, cost more as that grows.
 // A 64x64 render at 4 spp takes 650 us with a wait per iteration, 423 with
-// chains of 4, 408 with 8 (442 without overlapped launches); 1M paths 1820,
-// 1758 and 1752. From 2M paths an iteration takes milliseconds and the wait
-// does not show.
+// chains of 4, 408 with 8 (442 without overlapped launches), 1M paths 1820, 1758
+// and 1752; chains of 16 equal those of 8. The limit is not critical: 2^19
+// paths instead of 2^20 changes renders of 0.25M to 4M paths (Cornell box, a
+// mesh) by -1.0 to +0.3%, 2^22 costs 1 to 3% from 1.1M to 1.5M paths and 3 to 9%
+// from 2M on.
 constexpr uint32_t kChain = 8;
 constexpr uint32_t kChainPaths = 1u << 20;
 
