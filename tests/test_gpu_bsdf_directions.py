@@ -18,7 +18,7 @@ def test_direction_alone_equals_the_sample(ctx, kind):
     wo = rng.normal(size=(n, 3))
     wo[::5, 2] *= 1e-3   # grazing, from either side
     wo[::17, 2] = 0.0    # in the surface
-    wo[::19, :2] = 0.0   # along the normal
+    wo[::19] = 0.0, 0.0, 1.0  # along the normal
     wo /= np.linalg.norm(wo, axis=1, keepdims=True)
     u = rng.uniform(size=(n, 3)).astype(np.float32)
     u[::23, 0], u[::29, 1], u[::31, 2] = 0.5, 0.5, 0.0
